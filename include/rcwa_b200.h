@@ -252,16 +252,17 @@ int rcwa_set_qr_sweep_limit(int sweeps);
 
 /* CTAs per matrix of the Hessenberg reduction and the multishift Schur
  * iteration (no reference counterpart: a scheduling choice of this engine).
- * A batch of large matrices (order >= 1024) that would leave half of the SMs
- * idle is given a thread-block cluster of up to 8 CTAs per matrix; every
- * element is computed by the same operations whatever the team size, so the
+ * A batch that would leave half of the SMs idle is given a thread-block
+ * cluster of up to 8 CTAs per matrix (orders of at most 116, which run in
+ * shared memory, one CTA); every element is computed by the same operations whatever the team size, so the
  * results are identical.  ctas = 0 restores the automatic choice, 1..8 forces
  * a size for every later eigensolve (matrices of order >= 64).  Process-wide;
  * a plan captured into a CUDA graph keeps the size chosen when it was
  * captured.  Returns RCWA_ERR_INVALID outside 0..8. */
 int rcwa_set_eig_cluster(int ctas);
 /* The team size rcwa_set_eig_cluster's setting gives a batch of `batch`
- * order-n matrices on the current device. */
+ * order-n matrices on the current device.  The automatic choice is reported
+ * from order 1024 on; smaller orders report 1. */
 int rcwa_eig_cluster_size(int n, int batch);
 /* The same for the panel step of the LU factorisations (interface and tau
  * factorisations, rcwa_zgetrf stages): a batch of large matrices (order >=
@@ -305,9 +306,10 @@ int rcwa_zgemm_batched(rcwa_engine* e, int M, int N, int K, int batch, const rcw
  *   RCWA_TUNE_LU       0: one CTA factors each matrix, 1: panel by panel,
  *                      2: 128-column blocks (1 inside each block, then one
  *                      K = 128 trailing update per block; n >= 256)
- *   RCWA_TUNE_SCHUR    active-block size below which the Schur iteration uses
- *                      single-shift sweeps (64, 96, 128, 192; only 64 for
- *                      n < 64 and n >= 512; default 128 for 64 <= n < 128,
+ *   RCWA_TUNE_SCHUR    order below which a matrix (of at most 116 rows) is
+ *                      brought to Schur form in shared memory instead of by
+ *                      windowed multishift sweeps (64, 96, 128, 192; only 64
+ *                      for n < 64 and n >= 512; default 128 for 64 <= n < 128,
  *                      else 64)
  *   RCWA_TUNE_PRODUCT  mixed plans' cascade products and their tile shape,
  *                      0: 3xTF32 on tcgen05 with 128 x 128 output tiles,

@@ -1,11 +1,10 @@
 // Batched complex eigensolver, one CTA per matrix, FP64 throughout:
 //   1. Householder reduction to upper Hessenberg form, Q accumulated backwards;
-//   2. single-shift complex QR iteration (Wilkinson shifts, exceptional shifts
-//      every 10 sweeps, Ahues-Tisseur deflation test) producing the Schur form
-//      T with Schur vectors Z.  The bulge is chased by one warp inside a
-//      32 x 32 window held in shared memory; the window's rotations are then
-//      applied to the rest of T and to Z by the whole CTA, each thread
-//      streaming one row or column through the whole rotation sequence;
+//   2. small-bulge multishift QR (Ahues-Tisseur deflation test, exceptional
+//      shifts after 10 sweeps) producing the Schur form T with Schur vectors Z:
+//      matrices of at most kBlkMax rows entirely in shared memory
+//      (schur_block), larger ones through a chase window in shared memory with
+//      aggressive early deflation (schur_ms);
 //   3. eigenvectors of T by back-substitution (protected small divisors),
 //      back-transformed with Z by the tile GEMM and normalised to unit 2-norm.
 // This replaces LAPACK zgeev('N','V') behind MKLEigenSolver
@@ -14,6 +13,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <tuple>
 
 #include "eig.cuh"
 #include "linalg.cuh"
@@ -23,7 +23,6 @@ namespace {
 
 constexpr int kEigThreads = kTileThreads;  // 256
 constexpr int kWin = 32;
-constexpr int kItsPerEig = 300;
 
 constexpr int kHb = kEigPanel;
 
@@ -33,7 +32,7 @@ struct Scratch {
   cplx* Z;     // n*n, column-major: Z(r, c) = Z[c*n + r]
   cplx* X;     // n*n, row-major upper-triangular eigenvector matrix of T
   cplx* v;     // n: current Householder vector / work column
-  cplx* wv;    // n
+  double* scale; // what the Schur form is to be multiplied with (n complex)
   cplx* uv;    // n
   cplx* v0;    // n: leading element of each stored reflector
   cplx* Vb;    // n x kHb  panel reflectors, explicit (row-major)
@@ -63,8 +62,8 @@ __device__ Scratch scratch_for(void* work, int n, int b) {
   s.Z = (cplx*)base;
   s.X = s.Z + nn;
   s.v = s.X + nn;
-  s.wv = s.v + n;
-  s.uv = s.wv + n;
+  s.scale = reinterpret_cast<double*>(s.v + n);
+  s.uv = s.v + 2 * (size_t)n;
   s.v0 = s.uv + n;
   s.Vb = s.v0 + n;
   s.VH = s.Vb + nk;
@@ -437,22 +436,42 @@ __device__ void hessenberg_blocked(cplx* A, int n, int lda, const Scratch& s, do
 }
 
 // ---------------------------------------------------------------- QR
-// Rotation [c s; -conj(s) c] (c real) with G [x; y] = [r; 0], evaluated
-// with two reciprocal square roots after scaling both inputs by a power of
-// two: c = |x| / |(x, y)|, s = x conj(y) / (|x| |(x, y)|).
-__device__ __forceinline__ void givens_fast(cplx x, cplx y, double& c, cplx& s) {
+// Rotation [c s; -conj(s) c] (c real) with G [x; y] = [r; 0]:
+// c = |x| / |(x, y)|, s = x conj(y) / (|x| |(x, y)|), from one reciprocal
+// square root of |x|^2 |(x, y)|^2 and a Newton step towards c^2 + |s|^2 = 1
+// (with it the residuals of the eigenpairs are 2-4% below, without it 9% above
+// those of two reciprocal square roots; random matrices of order 40-450).
+// Inputs whose squares could leave the normal range are scaled by a power of
+// two first (exact), out of line: the scaling alone (frexp, ldexp) takes as
+// many cycles as the rest of the rotation, which is the serial step of every
+// QR sweep.
+__device__ __noinline__ void givens_scaled(cplx x, cplx y, double& c, cplx& s) {
+  if (y.x == 0.0 && y.y == 0.0) { c = 1.0; s = mkc(0.0, 0.0); return; }
   const double m = fmax(fmax(fabs(x.x), fabs(x.y)), fmax(fabs(y.x), fabs(y.y)));
-  if (m == 0.0 || (y.x == 0.0 && y.y == 0.0)) { c = 1.0; s = mkc(0.0, 0.0); return; }
   int e;
   frexp(m, &e);
   const double sc = ldexp(1.0, -e);
   x = cscale(x, sc);
   y = cscale(y, sc);
-  const double ax2 = cnorm2(x), ay2 = cnorm2(y);
+  const double ax2 = cnorm2(x);
   if (ax2 == 0.0) { c = 0.0; s = mkc(1.0, 0.0); return; }
-  const double ra = rsqrt(ax2), rr = rsqrt(ax2 + ay2);
+  const double ra = rsqrt(ax2), rr = rsqrt(ax2 + cnorm2(y));
   c = ax2 * ra * rr;
   s = cscale(cmul(x, cconj(y)), ra * rr);
+}
+__device__ __forceinline__ void givens_fast(cplx x, cplx y, double& c, cplx& s) {
+  const double ax2 = cnorm2(x), r2 = ax2 + cnorm2(y);
+  if (ax2 > 0x1p-400 && r2 < 0x1p400) {
+    const double q = rsqrt(ax2 * r2);
+    c = ax2 * q;
+    s = cscale(cmul(x, cconj(y)), q);
+    // one Newton step towards c^2 + |s|^2 = 1
+    const double h = 0.5 * fma(-s.y, s.y, fma(-s.x, s.x, fma(-c, c, 1.0)));
+    c = fma(c, h, c);
+    s = mkc(fma(s.x, h, s.x), fma(s.y, h, s.y));
+  } else {
+    givens_scaled(x, y, c, s);
+  }
 }
 
 // Negligible subdiagonal T(k,k-1) inside the active block [l, i]:
@@ -592,79 +611,200 @@ __device__ void qr_sweep(cplx* T, int ldt, cplx* Z, int n, int l, int i, cplx sh
   }
 }
 
-// Returns 0 or RCWA_ERR_NOCONV.
-__device__ int schur(cplx* T, int ldt, cplx* Z, int n, cplx (*Wt)[kWin + 1], double* rc, cplx* rs,
-                     int* redi, int sweep_cap) {
+// ---------------------------------------------------------------- Schur form of a small matrix
+// Matrices of at most kBlkMax rows: the whole matrix in shared memory, small-
+// bulge multishift sweeps of up to kBlkShifts bulges three rows apart, two
+// warps per bulge.  The first evaluates the rotation (every lane the same
+// arithmetic on a broadcast read) and updates the bulge's rows of T, then
+// after a barrier its columns, while the second applies the previous barrier's
+// rotation to the Schur vectors: a chain passes column p + 1 from one rotation
+// to the next in registers and fetches column p + 2 a step ahead, so Z stays
+// in global memory (L1/L2) and leaves the shared memory to T (5 CTAs per SM at
+// order 50).  The shifts are the two eigenvalues of the trailing 2 x 2 block; a
+// sweep of four uses each twice (near convergence the second pair still gains
+// a factor of the error, and it costs no extra steps).
+//
+// Bound by the serial latency of a chain step (the rotation, two barriers),
+// which this pays once for up to kBlkShifts rotations and without memory in
+// the chain; single-shift sweeps over a 32-row window with the rest of T and
+// Z updated in global memory took 2.58 ms for one matrix of order 50 (B200).
+constexpr int kBlkMax = 116;
+constexpr int kBlkShifts = 4;
+constexpr int kBlkThreads = 64 * kBlkShifts;
+
+__host__ __device__ constexpr int blk_ld(int n) { return n | 1; }  // odd pitch: conflict-free columns
+constexpr size_t blk_smem(int n) { return sizeof(cplx) * (size_t)n * blk_ld(n); }
+static_assert(blk_smem(kBlkMax) <= 230000, "the block must fit beside the kernel's static shared memory");
+
+// T: n x n upper Hessenberg in shared memory, pitch ld; Z: column-major in
+// global memory (Z(r, c) = Z[c*n + r]); n <= 32 Q.  Whole CTA; every warp takes
+// the same decisions from the same data.  Returns 0 or RCWA_ERR_NOCONV.
+template <int Q>
+__device__ int schur_block(cplx* T, int ld, cplx* Z, int n, int sweep_cap) {
+  __shared__ cplx s_sn[kBlkShifts];
+  __shared__ double s_c[kBlkShifts];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int b = warp >> 1;            // this warp's bulge
+  const bool lead = (warp & 1) == 0;  // rotation and T; else Z
   const double ulp = 2.0 * RCWA_DBL_EPS;
   const double smlnum = RCWA_DBL_MIN * ((double)n / ulp);
-  int i = n - 1;
-  long long total = 0;
-  const long long itmax_total = sweep_cap > 0 ? min(30LL * max(10, n), (long long)sweep_cap) : 30LL * max(10, n);
-  while (i >= 0) {
-    int l = 0;
-    bool conv = false;
-    for (int its = 0; its <= kItsPerEig; ++its) {
-      int best = l;
-      for (int k = l + 1 + threadIdx.x; k <= i; k += blockDim.x)
-        if (negligible(T, ldt, k, l, i, ulp, smlnum)) best = max(best, k);
-      l = block_max_int(best, redi);
-      if (l > 0 && threadIdx.x == 0) T[(size_t)l * ldt + l - 1] = mkc(0.0, 0.0);
-      __syncthreads();
-      if (l >= i) { conv = true; break; }
-      cplx shift;
-      if (its == 10 || its == 30) {
-        shift = cadd(T[(size_t)l * ldt + l], mkc(0.75 * cabs1(T[(size_t)(l + 1) * ldt + l]), 0.0));
-      } else if (its == 20 || its == 40) {
-        shift = cadd(T[(size_t)i * ldt + i], mkc(0.75 * cabs1(T[(size_t)i * ldt + i - 1]), 0.0));
-      } else {
-        shift = wilkinson_shift(T[(size_t)(i - 1) * ldt + i - 1], T[(size_t)(i - 1) * ldt + i],
-                                T[(size_t)i * ldt + i - 1], T[(size_t)i * ldt + i]);
+  const int budget = sweep_cap > 0 ? min(30 * max(10, n), sweep_cap) : 30 * max(10, n);
+  int hi = n - 1, its = 0;
+  for (int total = 0; hi >= 0;) {
+    __syncthreads();
+    int lo = 0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int k = lane + 32 * q;
+      const unsigned m = __ballot_sync(0xffffffffu, k >= 1 && k <= hi && negligible(T, ld, k, 0, hi, ulp, smlnum));
+      if (m) lo = 32 * q + 31 - __clz(m);
+    }
+    // every warp has read the subdiagonal before one thread clears an entry
+    __syncthreads();
+    if (lo > 0 && threadIdx.x == 0) T[lo * ld + lo - 1] = mkc(0.0, 0.0);
+    if (lo == hi) {
+      --hi;
+      its = 0;
+      continue;
+    }
+    if (++total > budget) return RCWA_ERR_NOCONV;
+    const int m = hi - lo + 1;
+    const int s = m < 4 ? 1 : m < 8 ? 2 : kBlkShifts;
+    cplx sh;
+    if (its == 10 || its == 30) {
+      sh = cadd(T[lo * ld + lo], mkc(0.75 * cabs1(T[(lo + 1) * ld + lo]), 0.0));
+    } else if (its == 20 || its == 40) {
+      sh = cadd(T[hi * ld + hi], mkc(0.75 * cabs1(T[hi * ld + hi - 1]), 0.0));
+    } else {
+      const cplx ta = T[(hi - 1) * ld + hi - 1], td = T[hi * ld + hi];
+      sh = wilkinson_shift(ta, T[(hi - 1) * ld + hi], T[hi * ld + hi - 1], td);
+      if (b & 1) sh = csub(cadd(ta, td), sh);  // the other eigenvalue
+    }
+    ++its;
+    __syncthreads();
+    const int tend = (hi - lo) + 3 * (s - 1);
+    cplx zx[Q], zy[Q];  // Z warps: columns p and p + 1
+#pragma unroll
+    for (int q = 0; q < Q; ++q) zx[q] = zy[q] = mkc(0.0, 0.0);
+    for (int t = 0; t < tend; ++t) {
+      const int p = lo + t - 3 * b;
+      const bool on = b < s && p >= lo && p <= hi - 1;
+      double c = 1.0;
+      cplx sn = mkc(0.0, 0.0);
+      if (lead) {
+        if (on) {
+          cplx* const r0 = T + p * ld;
+          cplx* const r1 = r0 + ld;
+          const int j0 = (p == lo ? p : p - 1) + lane;
+          cplx x, y, ra[Q], rb[Q];
+          if (p == lo) { x = csub(r0[p], sh); y = r1[p]; }
+          else { x = r0[p - 1]; y = r1[p - 1]; }
+#pragma unroll
+          for (int q = 0; q < Q; ++q)
+            if (j0 + 32 * q < n) { ra[q] = r0[j0 + 32 * q]; rb[q] = r1[j0 + 32 * q]; }
+          givens_fast(x, y, c, sn);
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const int j = j0 + 32 * q;
+            if (j < n) {
+              r0[j] = cfma(sn, rb[q], cscale(ra[q], c));
+              r1[j] = j < p ? mkc(0.0, 0.0) : cfma(cneg(cconj(sn)), ra[q], cscale(rb[q], c));
+            }
+          }
+          if (lane == 0) { s_c[b] = c; s_sn[b] = sn; }
+        }
+      } else if (b < s && p == lo) {
+        // the bulge behind left these columns two and three steps ago
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          if (lane + 32 * q < n) {
+            zx[q] = Z[(size_t)p * n + lane + 32 * q];
+            zy[q] = Z[(size_t)(p + 1) * n + lane + 32 * q];
+          }
       }
       __syncthreads();
-      qr_sweep(T, ldt, Z, n, l, i, shift, Wt, rc, rs);
-      if (++total > itmax_total) break;
+      if (on) {
+        if (lead) {
+          cplx* const col = T + p;
+          const int rn = min(p + 2, hi);
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const int r = lane + 32 * q;
+            if (r <= rn) {
+              const cplx x = col[r * ld], y = col[r * ld + 1];
+              col[r * ld] = cfma(cconj(sn), y, cscale(x, c));
+              col[r * ld + 1] = cfma(cneg(sn), x, cscale(y, c));
+            }
+          }
+        } else {
+          c = s_c[b];
+          sn = s_sn[b];
+          const bool last = p == hi - 1;
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const int r = lane + 32 * q;
+            if (r < n) {
+              Z[(size_t)p * n + r] = cfma(cconj(sn), zy[q], cscale(zx[q], c));
+              zx[q] = cfma(cneg(sn), zx[q], cscale(zy[q], c));
+              if (last) Z[(size_t)(p + 1) * n + r] = zx[q];
+              else zy[q] = Z[(size_t)(p + 2) * n + r];
+            }
+          }
+        }
+      }
+      __syncthreads();
     }
-    if (!conv) return RCWA_ERR_NOCONV;
-    i = l - 1;
   }
+  __syncthreads();
   return 0;
 }
-
 
 // ---------------------------------------------------------------- multishift QR
 // Small-bulge multishift QR (the scheme of Braman, Byers and Mathias, SIAM J.
 // Matrix Anal. Appl. 23(4), 2002) for complex Hessenberg matrices.  A sweep
 // chases a chain of s single-shift bulges, three rows apart, from the top to
-// the bottom of the active block.  The chain advances inside a 64 x 64 window
-// held in shared memory, all bulges of one chain step in parallel (their row
-// pairs and column pairs are disjoint).  Every rotation is logged; after a
-// window pass the log is applied to the rest of T (the rows right of the
-// window, the columns above it) and to Z, one line of 32 per warp task, with
-// the part of each line the chain spans held in registers (replay_frame), so
-// an element of T or Z crosses memory once per pass instead of once per
-// rotation.
+// the bottom of the active block.  The chain advances inside a W x W window
+// held in shared memory, one warp per bulge (their row pairs and column pairs
+// are disjoint), so a chain step costs two barriers.  Every rotation is
+// logged; after a window pass the log is applied to the rest of T (the rows
+// right of the window, the columns above it) and to Z, one line of 32 per
+// warp task, with the part of each line the chain spans held in registers
+// (replay_frame), so an element of T or Z crosses memory once per pass
+// instead of once per rotation.
+//
+// What bounds it (order 882, one matrix per SM, cycle counters of a lone
+// matrix, 64-row window and 16-row early deflation): the replay 191 of 298 ms,
+// at 7.0 cycles per rotation of 32 lines and SM against 6 of its eight
+// FP64 instructions alone; then the serial latency of the chase (51 ms) and of
+// the early deflation (54 ms).  With every rotation at 12 FP64 instructions, a
+// register shift per step and the chase's rotations on ten threads the same
+// matrix took 404 ms.  Schur stage of whole batches (window 64 / 72 / 100, early
+// deflation 16): 145 x 882 335 / 325 / 372 ms, 148 x 450 80 / 78 / 89 ms; ten
+// shifts (the frame spills) 537 ms, six 468 ms at 145 x 882.
 #ifndef RCWA_MS_WINDOW
-#define RCWA_MS_WINDOW 64
+#define RCWA_MS_WINDOW 72
 #endif
 constexpr int kMsW = RCWA_MS_WINDOW;  // window order (a build-time parameter)
 #ifndef RCWA_MS_SHIFTS
-#define RCWA_MS_SHIFTS 10
+#define RCWA_MS_SHIFTS 8
 #endif
 constexpr int kMsShifts = RCWA_MS_SHIFTS;  // bulges per sweep (a build-time parameter)
-constexpr int kMsMin = kSchurCrossover;  // smallest crossover: the chase window needs 64 rows
-constexpr int kMsThreads = 256;    // eight warps
-constexpr int kMsLog = kMsW + 1;         // rotation log per bulge; slot kMsW holds the identity
-constexpr int kMsMaxSteps = kMsW + 3 * kMsShifts;  // chain steps of one window pass
+constexpr int kMsMin = kSchurCrossover;  // smallest crossover
+constexpr int kMsThreads = 32 * kMsShifts;  // a warp per bulge in the chase, all of them in the replay
+constexpr int kMsLd = kMsW + 1;
+constexpr int kMsFrame = 3 * (kMsShifts - 1) + 2;  // indices the chain spans
+constexpr int kMsPre = 4;                          // replay steps per unrolled group
+// chain steps of one window pass, rounded up to whole replay groups
+constexpr int kMsMaxSteps = (kMsW + 3 * kMsShifts + kMsPre - 1) / kMsPre * kMsPre;
+static_assert(kMsW % 2 == 0, "an odd window pitch keeps column accesses conflict free");
 
 struct MsSmem {
-  cplx* Wt;      // [kMsW][kMsW + 1]  the chase window
+  cplx* Wt;      // [kMsW][kMsLd]  the chase window
   cplx* work;    // early deflation's window, vectors and reflector; the small shift problem
-  double* lc;    // [kMsShifts][kMsLog]  rotation cosines, bulge-major
-  cplx* ls;      // [kMsShifts][kMsLog]  rotation sines
-  int* ix;       // [kMsMaxSteps][kMsShifts]  log slot per chain step and bulge
-  int* firstp;   // [kMsShifts] first rotation position of each bulge in the pass
-  int* cnt;      // [kMsShifts] rotations of each bulge in the pass
-  int* tfirst;   // [kMsShifts] pass step of each bulge's first rotation
+  cplx* log;     // [kMsMaxSteps][kMsShifts][2]  replay coefficients per chain step and bulge
+  double* lc;    // [kMsMaxSteps][kMsShifts]  rotation cosines
+  double* dfin;  // [kMsW]  scale of every window index after the pass
   cplx* shifts;  // [kMsShifts]
   int* redi;     // [kMsThreads / 32]
   int* aed;      // [4] early-deflation results: converged flag, undeflated count, shift count
@@ -672,30 +812,30 @@ struct MsSmem {
 
 // the window is only used by the chase, the work area only by the early
 // deflation and the shift computation between sweeps: they share one region
-constexpr size_t kMsRegion = sizeof(cplx) * kMsW * (kMsW + 1);
-constexpr size_t kMsSmemBytes = kMsRegion +
-                                sizeof(double) * kMsShifts * kMsLog + sizeof(cplx) * kMsShifts * kMsLog +
-                                sizeof(int) * kMsMaxSteps * kMsShifts + sizeof(int) * 3 * kMsShifts +
-                                sizeof(cplx) * kMsShifts + sizeof(int) * (kMsThreads / 32 + 4);
+constexpr size_t kMsRegion = sizeof(cplx) * kMsW * kMsLd;
+constexpr size_t kMsSmemBytes = kMsRegion + 2 * sizeof(cplx) * kMsMaxSteps * kMsShifts +
+                                sizeof(double) * (kMsMaxSteps * kMsShifts + kMsW) + sizeof(cplx) * kMsShifts +
+                                sizeof(int) * (kMsThreads / 32 + 4);
 static_assert(kMsSmemBytes <= 232448, "multishift shared memory exceeds the per-block limit");
 
 __device__ MsSmem carve_ms_smem(unsigned char* base) {
   MsSmem sm;
   sm.Wt = (cplx*)base;
   sm.work = (cplx*)base;
-  sm.ls = (cplx*)(base + kMsRegion);
-  sm.shifts = sm.ls + kMsShifts * kMsLog;
+  sm.log = (cplx*)(base + kMsRegion);
+  sm.shifts = sm.log + 2 * kMsMaxSteps * kMsShifts;
   sm.lc = (double*)(sm.shifts + kMsShifts);
-  sm.ix = (int*)(sm.lc + kMsShifts * kMsLog);
-  sm.firstp = sm.ix + kMsMaxSteps * kMsShifts;
-  sm.cnt = sm.firstp + kMsShifts;
-  sm.tfirst = sm.cnt + kMsShifts;
-  sm.redi = sm.tfirst + kMsShifts;
+  sm.dfin = sm.lc + kMsMaxSteps * kMsShifts;
+  sm.redi = (int*)(sm.dfin + kMsW);
   sm.aed = sm.redi + kMsThreads / 32;
   return sm;
 }
 
-#define MSW(r, c) sm.Wt[(r) * (kMsW + 1) + (c)]
+// the multishift kernel's dynamic shared memory (the replay is a function of
+// its own, so that its frame has the registers to itself)
+extern __shared__ __align__(16) unsigned char ms_dsm[];
+
+#define MSW(r, c) sm.Wt[(r) * kMsLd + (c)]
 
 // Eigenvalues of the s x s upper Hessenberg matrix B (row stride ldb) by
 // single-shift QR without vectors; one warp.  Unconverged remainders after
@@ -760,30 +900,33 @@ __device__ void small_eigs_warp(cplx* B, int ldb, int s, cplx* out) {
 // deflated, the others are moved to the top by adjacent swaps and serve as
 // shifts; the spike of the undeflated part is reflected onto its first entry
 // and that part is returned to Hessenberg form by Householder reflectors.
-// Measured on the cfg2 FP64 step (740 matrices of 882): Schur 2488 / 2286 /
-// 2251 / 2228 / 2260 / 2251 ms with windows of 32 / 20 / 18 / 16 / 14 / 12
-// (a smaller window's cheaper one-warp Schur against its fewer deflations);
-// with 16, 8 and 12 shifts per sweep gave 2271 and 2231 ms against 2228.
+// The window's one-warp Schur form is serial, so a smaller window is cheaper
+// per call and deflates less: Schur stage with windows of 16 / 14 / 12 (64-row
+// chase window) 145 x 882 335 / 346 / 342 ms, 148 x 450 80 / 81 / 75 ms, 74 x
+// 198 19.6 / 18.8 / 16.3 ms; a 32-row window on all warps cut the sweeps by 20%
+// but cost 60 + 35 ms for its Schur form and reordering at order 882.
 #ifndef RCWA_AED_WINDOW
-#define RCWA_AED_WINDOW 16
+#define RCWA_AED_WINDOW 12
 #endif
-constexpr int kAedW = RCWA_AED_WINDOW;  // window order (one lane per column; a build-time parameter)
-static_assert(kAedW <= 32 && kAedW >= kMsShifts + 2, "the early-deflation window is one warp wide");
+constexpr int kAedW = RCWA_AED_WINDOW;  // window order (a build-time parameter)
+static_assert(kAedW <= 16 && kAedW >= kMsShifts + 2, "a half warp per row of the early-deflation window and of V");
 constexpr int kAedLd = kAedW + 1;
 constexpr int kAedNibble = 14;   // percent of the window deflated that skips the sweep
 static_assert(sizeof(cplx) * (2 * kAedW * kAedLd + kAedW) <= kMsRegion &&
-                  sizeof(cplx) * kMsShifts * (kMsShifts + 1) <= kMsRegion,
-              "the early-deflation work area must fit in the chase window's region");
+                  sizeof(cplx) * kMsShifts * (kMsShifts + 1) <= kMsRegion && sizeof(cplx) * kWin * (kWin + 1) <= kMsRegion,
+              "the work areas must fit in the chase window's region");
 
 #define AW(r, c) W[(r) * kAedLd + (c)]
 #define AV(r, c) V[(r) * kAedLd + (c)]
 
 // Schur form of the Hessenberg window W (nw x nw) with V <- V G^H for every
-// rotation G; single-shift QR by one warp.  Returns false when the iteration
-// budget runs out.
+// rotation G; single-shift QR by one warp, lanes 0-15 on W and lanes 16-31 on
+// V.  Returns false when the iteration budget runs out.
 __device__ bool aed_window_schur(cplx* W, cplx* V, int nw) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, idx = lane & 15;
+  const bool wl = lane < 16;
   const double ulp = 2.0 * RCWA_DBL_EPS;
+  cplx* const col = wl ? W : V;  // this lane's row of W or V in the column updates
   int hi = nw - 1, its = 0, total = 0;
   while (hi >= 0) {
     __syncwarp();
@@ -812,26 +955,23 @@ __device__ bool aed_window_schur(cplx* W, cplx* V, int nw) {
       cplx x, y;
       if (p == lo) { x = csub(AW(lo, lo), sh); y = AW(lo + 1, lo); }
       else { x = AW(p, p - 1); y = AW(p + 1, p - 1); }
+      const bool row = wl && idx >= (p == lo ? p : p - 1) && idx < nw;
+      cplx a = mkc(0.0, 0.0), b = mkc(0.0, 0.0);
+      if (row) { a = AW(p, idx); b = AW(p + 1, idx); }
       double c;
       cplx sn;
       givens_fast(x, y, c, sn);
       __syncwarp();
-      if (lane >= (p == lo ? p : p - 1) && lane < nw) {
-        const cplx a = AW(p, lane), b = AW(p + 1, lane);
-        AW(p, lane) = cfma(sn, b, cscale(a, c));
-        AW(p + 1, lane) = cfma(cneg(cconj(sn)), a, cscale(b, c));
+      if (row) {
+        AW(p, idx) = cfma(sn, b, cscale(a, c));
+        AW(p + 1, idx) = idx < p ? mkc(0.0, 0.0) : cfma(cneg(cconj(sn)), a, cscale(b, c));
       }
       __syncwarp();
-      if (p > lo && lane == 0) AW(p + 1, p - 1) = mkc(0.0, 0.0);
-      if (lane <= min(p + 2, hi)) {
-        const cplx a = AW(lane, p), b = AW(lane, p + 1);
-        AW(lane, p) = cfma(cconj(sn), b, cscale(a, c));
-        AW(lane, p + 1) = cfma(cneg(sn), a, cscale(b, c));
-      }
-      if (lane < nw) {
-        const cplx a = AV(lane, p), b = AV(lane, p + 1);
-        AV(lane, p) = cfma(cconj(sn), b, cscale(a, c));
-        AV(lane, p + 1) = cfma(cneg(sn), a, cscale(b, c));
+      if (idx <= (wl ? min(p + 2, hi) : nw - 1)) {
+        a = col[idx * kAedLd + p];
+        b = col[idx * kAedLd + p + 1];
+        col[idx * kAedLd + p] = cfma(cconj(sn), b, cscale(a, c));
+        col[idx * kAedLd + p + 1] = cfma(cneg(sn), a, cscale(b, c));
       }
       __syncwarp();
     }
@@ -844,28 +984,25 @@ __device__ bool aed_window_schur(cplx* W, cplx* V, int nw) {
 // Swap the adjacent eigenvalues k, k+1 of the upper triangular W (LAPACK
 // ztrexc step): G from (W(k,k+1), W(k+1,k+1) - W(k,k)) applied to rows
 // k, k+1 right of the pair, to columns k, k+1 above it and to V; the
-// diagonal entries trade places and W(k,k+1) keeps its value.  One warp.
+// diagonal entries trade places and W(k,k+1) keeps its value.  One warp: the
+// three updates touch disjoint entries, lanes 0-15 take those of W and lanes
+// 16-31 those of V.
 __device__ void aed_swap(cplx* W, cplx* V, int nw, int k) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, idx = lane & 15;
+  const bool wl = lane < 16, row = wl && idx >= k + 2 && idx < nw, cl = wl ? idx < k : idx < nw;
+  cplx* const pa = row ? &AW(k, idx) : wl ? &AW(idx, k) : &AV(idx, k);
+  cplx* const pb = row ? &AW(k + 1, idx) : pa + 1;
   const cplx t11 = AW(k, k), t22 = AW(k + 1, k + 1);
+  cplx a = mkc(0.0, 0.0), b = mkc(0.0, 0.0);
+  if (row || cl) { a = *pa; b = *pb; }
   double c;
   cplx sn;
   givens_fast(AW(k, k + 1), csub(t22, t11), c, sn);
   __syncwarp();
-  if (lane >= k + 2 && lane < nw) {
-    const cplx a = AW(k, lane), b = AW(k + 1, lane);
-    AW(k, lane) = cfma(sn, b, cscale(a, c));
-    AW(k + 1, lane) = cfma(cneg(cconj(sn)), a, cscale(b, c));
-  }
-  if (lane < k) {
-    const cplx a = AW(lane, k), b = AW(lane, k + 1);
-    AW(lane, k) = cfma(cconj(sn), b, cscale(a, c));
-    AW(lane, k + 1) = cfma(cneg(sn), a, cscale(b, c));
-  }
-  if (lane < nw) {
-    const cplx a = AV(lane, k), b = AV(lane, k + 1);
-    AV(lane, k) = cfma(cconj(sn), b, cscale(a, c));
-    AV(lane, k + 1) = cfma(cneg(sn), a, cscale(b, c));
+  if (!row) sn = cconj(sn);
+  if (row || cl) {
+    *pa = cfma(sn, b, cscale(a, c));
+    *pb = cfma(cneg(cconj(sn)), a, cscale(b, c));
   }
   if (lane == 0) { AW(k, k) = t22; AW(k + 1, k + 1) = t11; }
   __syncwarp();
@@ -920,8 +1057,9 @@ __device__ void aed_right(cplx* M, const cplx* v, int len, cplx tau, int rows, i
   __syncwarp();
 }
 
-// Aggressive early deflation on the active block [l, i] (i - l + 1 > kAedW + 1).
-// Returns the number of deflated eigenvalues (0 when none, -1 when the window
+// Aggressive early deflation on the active block [l, i].  A block of at most
+// kAedW rows is the window itself: it has no spike, so its Schur form deflates
+// all of it.  Returns the number of deflated eigenvalues (0 when none, -1 when the window
 // did not converge and nothing was changed).  On return sm.shifts[0..cnt)
 // hold the bottom undeflated window eigenvalues, cnt <= kMsShifts, in
 // sm.aed[2].  Whole CTA.
@@ -935,19 +1073,19 @@ __device__ int aed(cplx* T, int ldt, cplx* Z, int n, int l, int i, const MsSmem&
   const int tid = threadIdx.x, nthr = blockDim.x;
   const bool lead = tm.rank == 0;
   const int stride = nthr * tm.size, off0 = tid + nthr * tm.rank;
-  const int nw = kAedW;
+  const int nw = min(kAedW, i - l + 1);
   const int kw = i - nw + 1;
   cplx* W = sm.work;
   cplx* V = W + kAedW * kAedLd;
   cplx* hv = V + kAedW * kAedLd;
   const double ulp = 2.0 * RCWA_DBL_EPS;
   const double smlnum = RCWA_DBL_MIN * ((double)n / ulp);
-  for (int idx = tid; idx < nw * nw; idx += nthr) {
-    const int r = idx / nw, c = idx % nw;
-    AW(r, c) = T[(size_t)(kw + r) * ldt + kw + c];
-    AV(r, c) = mkc(r == c ? 1.0 : 0.0, 0.0);
+  for (int idx = tid; idx < kAedW * kAedW; idx += nthr) {
+    const int r = idx / kAedW, c = idx % kAedW;
+    if (r < nw && c < nw) AW(r, c) = T[(size_t)(kw + r) * ldt + kw + c];
+    AV(r, c) = mkc(r == c && r < nw ? 1.0 : 0.0, 0.0);
   }
-  const cplx s = T[(size_t)kw * ldt + kw - 1];
+  const cplx s = kw > l ? T[(size_t)kw * ldt + kw - 1] : mkc(0.0, 0.0);
   __syncthreads();
   // every CTA holds the window before the first one writes it back
   if (tm.size > 1) tm.sync();
@@ -1036,19 +1174,19 @@ __device__ int aed(cplx* T, int ldt, cplx* Z, int n, int l, int i, const MsSmem&
 #endif
   // window, spike and the off-window blocks
   if (lead) {
-    for (int idx = tid; idx < nw * nw; idx += nthr) {
-      const int r = idx / nw, c = idx % nw;
-      T[(size_t)(kw + r) * ldt + kw + c] = AW(r, c);
+    for (int idx = tid; idx < kAedW * kAedW; idx += nthr) {
+      const int r = idx / kAedW, c = idx % kAedW;
+      if (r < nw && c < nw) T[(size_t)(kw + r) * ldt + kw + c] = AW(r, c);
     }
-    if (tid == 0) T[(size_t)kw * ldt + kw - 1] = cmul(s, cconj(AV(0, 0)));
+    if (tid == 0 && kw > l) T[(size_t)kw * ldt + kw - 1] = cmul(s, cconj(AV(0, 0)));
   }
   // rows kw..i right of the window: Vh * T
   for (int j = i + 1 + off0; j < n; j += stride) {
     cplx x[kAedW];
 #pragma unroll
-    for (int r = 0; r < kAedW; ++r) x[r] = T[(size_t)(kw + r) * ldt + j];
-#pragma unroll 4
-    for (int r = 0; r < kAedW; ++r) {
+    for (int r = 0; r < kAedW; ++r) x[r] = r < nw ? T[(size_t)(kw + r) * ldt + j] : mkc(0.0, 0.0);
+#pragma unroll 2
+    for (int r = 0; r < nw; ++r) {
       cplx acc = mkc(0.0, 0.0);
 #pragma unroll
       for (int c = 0; c < kAedW; ++c) acc = cfmaconj(AV(c, r), x[c], acc);
@@ -1059,9 +1197,9 @@ __device__ int aed(cplx* T, int ldt, cplx* Z, int n, int l, int i, const MsSmem&
   for (int r = off0; r < kw; r += stride) {
     cplx x[kAedW];
 #pragma unroll
-    for (int c = 0; c < kAedW; ++c) x[c] = T[(size_t)r * ldt + kw + c];
-#pragma unroll 4
-    for (int c = 0; c < kAedW; ++c) {
+    for (int c = 0; c < kAedW; ++c) x[c] = c < nw ? T[(size_t)r * ldt + kw + c] : mkc(0.0, 0.0);
+#pragma unroll 2
+    for (int c = 0; c < nw; ++c) {
       cplx acc = mkc(0.0, 0.0);
 #pragma unroll
       for (int k = 0; k < kAedW; ++k) acc = cfma(x[k], AV(k, c), acc);
@@ -1072,9 +1210,9 @@ __device__ int aed(cplx* T, int ldt, cplx* Z, int n, int l, int i, const MsSmem&
   for (int r = off0; r < n; r += stride) {
     cplx x[kAedW];
 #pragma unroll
-    for (int c = 0; c < kAedW; ++c) x[c] = Z[(size_t)(kw + c) * n + r];
-#pragma unroll 4
-    for (int c = 0; c < kAedW; ++c) {
+    for (int c = 0; c < kAedW; ++c) x[c] = c < nw ? Z[(size_t)(kw + c) * n + r] : mkc(0.0, 0.0);
+#pragma unroll 2
+    for (int c = 0; c < nw; ++c) {
       cplx acc = mkc(0.0, 0.0);
 #pragma unroll
       for (int k = 0; k < kAedW; ++k) acc = cfma(x[k], AV(k, c), acc);
@@ -1097,82 +1235,167 @@ __device__ int aed(cplx* T, int ldt, cplx* Z, int n, int l, int i, const MsSmem&
 // base + r * stride for index r in [rlo, rhi].  At pass step sg bulge b acts
 // on the pair (p, p+1), p = top0 + sg + 3 (kMsShifts - 1 - b), so the chain
 // spans kMsFrame consecutive indices that slide by one per step.  That span
-// is held in registers: each step loads the index entering at the bottom
-// (kMsPre steps ahead), applies the kMsShifts rotations in registers and
-// stores the index leaving at the top, so every element crosses memory once
-// per pass and the rotations run from registers, not shared memory.
+// is held in registers: each step takes in the index entering at the bottom
+// (loaded kMsPre steps ahead), applies the kMsShifts rotations and stores the
+// index leaving at the top, so every element crosses memory once per pass.
+// kMsPre steps are unrolled into one group over a frame of kMsFrame + kMsPre -
+// 1 registers, which then moves down by kMsPre in one go (a shift per step
+// cost as many moves as the rotations cost FP64 instructions).  nsteps is a
+// multiple of kMsPre (the log is padded with identities).
+//
 // Rows: [x; y] <- [c x + s y; -conj(s) x + c y]; columns: the conjugate
-// transpose [c x + conj(s) y; -s x + c y].
-constexpr int kMsFrame = 3 * (kMsShifts - 1) + 2;
-constexpr int kMsPre = 4;
-
-template <bool kRows>
-__device__ __forceinline__ void replay_frame(cplx* base, size_t stride, int top0, int nsteps, int rlo, int rhi,
-                                             const MsSmem& sm) {
-  cplx f[kMsFrame];
+// transpose [c x + conj(s) y; -s x + c y].  kScaled: the cosines are taken out
+// of the rotations (fast Givens rotations, W. M. Gentleman, J. Inst. Math.
+// Appl. 12, 1973): a register holds X with the true value x = d X, and with t
+// = s / c the pair becomes X + (t dy/dx) Y, Y - (conj(t) dx/dy) X with both
+// scales multiplied by c.  The two coefficients and the final scale of every
+// index are common to all lines and come from the log, so a rotation takes 8
+// FP64 instructions instead of 12; an element is scaled once, on leaving.
+template <bool kRows, bool kScaled>
+__device__ __noinline__ void replay_frame(cplx* base, int stride, int top0, int nsteps, int ws, int rlo, int rhi) {
+  cplx f[kMsFrame + kMsPre - 1];
+  const int lo = rlo - top0, hi = rhi - top0;  // [lo, hi]: the touched indices relative to top0
+  // walking pointers of the next entering and the next leaving element
+  cplx* out = base + (ptrdiff_t)top0 * stride;
+  const cplx* in = out;
 #pragma unroll
   for (int k = 0; k < kMsFrame - 1; ++k) {
-    const int r = top0 + k;
-    f[k] = (r >= rlo && r <= rhi) ? base[(size_t)r * stride] : mkc(0.0, 0.0);
+    f[k] = (k >= lo && k <= hi) ? *in : mkc(0.0, 0.0);
+    in += stride;
   }
-  f[kMsFrame - 1] = mkc(0.0, 0.0);
   cplx pre[kMsPre];
 #pragma unroll
   for (int d = 0; d < kMsPre; ++d) {
-    const int r = top0 + d + kMsFrame - 1;
-    pre[d] = (d < nsteps && r >= rlo && r <= rhi) ? base[(size_t)r * stride] : mkc(0.0, 0.0);
+    const int k = d + kMsFrame - 1;
+    pre[d] = (k >= lo && k <= hi) ? *in : mkc(0.0, 0.0);
+    in += stride;
   }
+  const MsSmem sm = carve_ms_smem(ms_dsm);
+  const cplx* e = sm.log;
+  const double* df = sm.dfin + (top0 - ws);
+#pragma unroll 1
   for (int sg0 = 0; sg0 < nsteps; sg0 += kMsPre) {
-    cplx cur[kMsPre];
 #pragma unroll
     for (int d = 0; d < kMsPre; ++d) {
-      cur[d] = pre[d];
-      const int sg = sg0 + kMsPre + d, r = top0 + sg + kMsFrame - 1;
-      pre[d] = (sg < nsteps && r >= rlo && r <= rhi) ? base[(size_t)r * stride] : mkc(0.0, 0.0);
+      f[kMsFrame - 1 + d] = pre[d];
+      const int k = sg0 + kMsPre + d + kMsFrame - 1;
+      pre[d] = (sg0 + kMsPre < nsteps && k >= lo && k <= hi) ? *in : mkc(0.0, 0.0);
+      in += stride;
     }
 #pragma unroll
     for (int d = 0; d < kMsPre; ++d) {
-      const int sg = sg0 + d;
-      if (sg < nsteps) {
-        f[kMsFrame - 1] = cur[d];
-        const int* e = sm.ix + sg * kMsShifts;
 #pragma unroll
-        for (int b = 0; b < kMsShifts; ++b) {
-          const int slot = e[b];
-          const double c = sm.lc[b * kMsLog + slot];
-          const cplx sn = sm.ls[b * kMsLog + slot];
-          const int kb = 3 * (kMsShifts - 1 - b);
-          const cplx x = f[kb], y = f[kb + 1];
-          if (kRows) {
-            f[kb] = cfma(sn, y, cscale(x, c));
-            f[kb + 1] = cfma(cneg(cconj(sn)), x, cscale(y, c));
-          } else {
-            f[kb] = cfma(cconj(sn), y, cscale(x, c));
-            f[kb + 1] = cfma(cneg(sn), x, cscale(y, c));
-          }
+      for (int b = 0; b < kMsShifts; ++b) {
+        const cplx e0 = e[2 * b], e1 = e[2 * b + 1];
+        const int kb = d + 3 * (kMsShifts - 1 - b);
+        const cplx x = f[kb], y = f[kb + 1];
+        if (kScaled) {
+          f[kb] = kRows ? cfma(e0, y, x) : cfmaconj(e0, y, x);
+          f[kb + 1] = kRows ? cfma(e1, x, y) : cfmaconj(e1, x, y);
+        } else {  // e0 = s, e1.x = c
+          f[kb] = kRows ? cfma(e0, y, cscale(x, e1.x)) : cfmaconj(e0, y, cscale(x, e1.x));
+          f[kb + 1] = cfma(cneg(kRows ? cconj(e0) : e0), x, cscale(y, e1.x));
         }
-        const int rt = top0 + sg;
-        if (rt >= rlo && rt <= rhi) base[(size_t)rt * stride] = f[0];
-#pragma unroll
-        for (int k = 0; k < kMsFrame - 1; ++k) f[k] = f[k + 1];
       }
+      e += 2 * kMsShifts;
+      const int k = sg0 + d;
+      if (k >= lo && k <= hi) *out = kScaled ? cscale(f[d], df[k]) : f[d];
+      out += stride;
+    }
+#pragma unroll
+    for (int k = 0; k < kMsFrame - 1; ++k) f[k] = f[k + kMsPre];
+  }
+#pragma unroll
+  for (int k0 = 0; k0 < kMsFrame - 1; ++k0) {
+    const int k = nsteps + k0;
+    if (k >= lo && k <= hi) *out = kScaled ? cscale(f[k0], df[k]) : f[k0];
+    out += stride;
+  }
+}
+
+// The lines a window pass leaves to the replay: columns of T right of the
+// window, rows of T above it, rows of Z, 32 lines per warp task, dealt over
+// the team's warps.
+template <bool kScaled>
+__device__ __forceinline__ void replay_lines(cplx* T, int ldt, cplx* Z, int n, int ws, int we, int top0, int nsteps,
+                                             int rlo, int rhi, const Team& tm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int nR = (n - 1 - we + 31) / 32, nU = (ws + 31) / 32, nZ = (n + 31) / 32;
+  for (int task = warp + nwarp * tm.rank; task < nR + nU + nZ; task += nwarp * tm.size) {
+    if (task < nR) {
+      // T(rlo..rhi, j), j right of the window: row rotations, lane = column
+      const int j = we + 1 + 32 * task + lane;
+      if (j < n) replay_frame<true, kScaled>(T + j, ldt, top0, nsteps, ws, rlo, rhi);
+    } else {
+      // T(r, rlo..rhi), r above the window (lane = row), or Z(r, rlo..rhi)
+      // (column-major, lane = row): column rotations
+      const bool up = task < nR + nU;
+      const int r = 32 * (up ? task - nR : task - nR - nU) + lane;
+      if (r < (up ? ws : n))
+        replay_frame<false, kScaled>(up ? T + (size_t)r * ldt : Z + r, up ? 1 : n, top0, nsteps, ws,
+                                     rlo, rhi);
     }
   }
-#pragma unroll
-  for (int k = 0; k < kMsFrame - 1; ++k) {
-    const int r = top0 + nsteps + k;
-    if (r >= rlo && r <= rhi) base[(size_t)r * stride] = f[k];
+}
+
+// Cosines below this keep a pass on the unscaled replay (the scaled one
+// divides by them; an index takes at most 2 kMsShifts rotations per pass, so
+// its scale stays above 2^-400).
+constexpr double kMsMinCos = 9.5367431640625e-07;  // 2^-20
+
+// The replay coefficients of a pass from its rotation log (cosines in lc,
+// sines in log[..][0]).  Index r takes, per bulge, the rotation at p = r - 1
+// as its second and the one at p = r as its first element; bulge b is at p
+// three steps after bulge b - 1.  So before bulge b's rotation at p (step sg)
+// the scales are products of the cosines of the earlier bulges at p - 1, p
+// and p + 1, all read from the log, and every entry is computed
+// independently.  Returns whether the scaled replay can be used.
+__device__ bool replay_coefficients(const MsSmem& sm, int top0, int ws, int nsteps) {
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  bool small = false;
+  for (int idx = tid; idx < nsteps * kMsShifts; idx += nthr) small |= sm.lc[idx] < kMsMinCos;
+  const bool scaled = !__syncthreads_or(small);
+  if (!scaled) {
+    for (int idx = tid; idx < nsteps * kMsShifts; idx += nthr) sm.log[2 * idx + 1] = mkc(sm.lc[idx], 0.0);
+    return false;
   }
+  auto cosine = [&](int sg, int b) { return sg >= 0 && sg < nsteps ? sm.lc[sg * kMsShifts + b] : 1.0; };
+  for (int idx = tid; idx < nsteps * kMsShifts; idx += nthr) {
+    const int sg = idx / kMsShifts, b = idx % kMsShifts;
+    double dx = cosine(sg - 1, b), dy = 1.0;
+    for (int q = 1; q <= b; ++q) {
+      const double c = cosine(sg - 3 * q, b - q);
+      dx *= cosine(sg - 3 * q - 1, b - q) * c;
+      dy *= cosine(sg - 3 * q + 1, b - q) * c;
+    }
+    const cplx s = sm.log[2 * idx];
+    const double c = sm.lc[idx], r = dy / (c * dx), q = dx / (c * dy);
+    sm.log[2 * idx] = cscale(s, r);
+    sm.log[2 * idx + 1] = mkc(-s.x * q, s.y * q);
+  }
+  // index r is at p = r at step r - top0 - 3 (kMsShifts - 1 - b) of bulge b
+  for (int r = tid; r < kMsW; r += nthr) {
+    double d = 1.0;
+    for (int b = 0; b < kMsShifts; ++b) {
+      const int sg = ws + r - top0 - 3 * (kMsShifts - 1 - b);
+      d *= cosine(sg - 1, b) * cosine(sg, b);
+    }
+    sm.dfin[r] = d;
+  }
+  return true;
 }
 
 // One multishift sweep over the active block [l, i] with sm.shifts[0..s).
 // Bulge b sits at position p = l + t - 3b at chain step t; it is active while
-// l <= p <= i-1 and its rotation acts on rows/columns (p, p+1).
+// l <= p <= i-1 and its rotation acts on rows/columns (p, p+1).  Warp b chases
+// bulge b: every lane evaluates the rotation (a broadcast read and the same
+// arithmetic, no exchange), then the warp updates the bulge's two rows, and
+// after a barrier its two columns.
 // With a team of several CTAs every CTA chases the bulges through its own
 // copy of the window (the same operations on the same data), the first CTA
 // writes the window back, and the off-window lines are split over the team.
 __device__ void ms_sweep(cplx* T, int ldt, cplx* Z, int n, int l, int i, int s, const MsSmem& sm, const Team& tm) {
-  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, b = tid >> 5;
   const int tend = (i - l) + 3 * (s - 1);
   int t = 0;
   while (t < tend) {
@@ -1193,65 +1416,67 @@ __device__ void ms_sweep(cplx* T, int ldt, cplx* Z, int n, int l, int i, int s, 
 #ifdef RCWA_EIG_STATS
     const long long c_start = clock64();
 #endif
-    if (tid < s) { sm.firstp[tid] = -1; sm.cnt[tid] = 0; }
     for (int idx = tid; idx < w * w; idx += nthr)
       cp_async16(&MSW(idx / w, idx % w), &T[(size_t)(ws + idx / w) * ldt + ws + idx % w]);
     cp_async_wait_all();
     __syncthreads();
     // every CTA holds its window before the first one writes it back
     if (tm.size > 1) tm.sync();
-    for (int tt = t; tt < t1; ++tt) {
-      const int over = l + tt - (i - 1);
-      const int bA = over > 0 ? (over + 2) / 3 : 0;
-      const int bB = min(s - 1, tt / 3);
-      if (tid >= bA && tid <= bB) {
-        const int b = tid, p = l + tt - 3 * b;
-        cplx x, y;
-        if (p == l) { x = csub(MSW(p - ws, p - ws), sm.shifts[b]); y = MSW(p + 1 - ws, p - ws); }
-        else { x = MSW(p - ws, p - 1 - ws); y = MSW(p + 1 - ws, p - 1 - ws); }
-        double c;
-        cplx sn;
+    const int nsteps = t1 - t;
+    for (int sg = 0; sg < nsteps; ++sg) {
+      const int p = l + t + sg - 3 * b;
+      const bool on = b < s && p >= l && p <= i - 1;
+      double c = 1.0;
+      cplx sn = mkc(0.0, 0.0);
+      if (on) {
+        cplx* const r0 = &MSW(p - ws, 0);
+        cplx* const r1 = r0 + kMsLd;
+        const int j0 = ((p == l) ? l : p - 1) - ws, jn = we - ws;
+        cplx x, y, ra[(kMsW + 31) / 32], rb[(kMsW + 31) / 32];
+        if (p == l) { x = csub(r0[p - ws], sm.shifts[b]); y = r1[p - ws]; }
+        else { x = r0[p - 1 - ws]; y = r1[p - 1 - ws]; }
+        // row operations: rows (p, p+1), columns max(p-1, l) .. we
+#pragma unroll
+        for (int q = 0; q < (kMsW + 31) / 32; ++q) {
+          const int j = j0 + lane + 32 * q;
+          if (j <= jn) { ra[q] = r0[j]; rb[q] = r1[j]; }
+        }
         givens_fast(x, y, c, sn);
-        if (sm.firstp[b] < 0) { sm.firstp[b] = p; sm.tfirst[b] = tt - t; }
-        const int k = p - sm.firstp[b];
-        sm.lc[b * kMsLog + k] = c;
-        sm.ls[b * kMsLog + k] = sn;
-        sm.cnt[b] = k + 1;
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < (kMsW + 31) / 32; ++q) {
+          const int j = j0 + lane + 32 * q;
+          if (j <= jn) {
+            r0[j] = cfma(sn, rb[q], cscale(ra[q], c));
+            r1[j] = j < p - ws ? mkc(0.0, 0.0) : cfma(cneg(cconj(sn)), ra[q], cscale(rb[q], c));
+          }
+        }
+      }
+      if (lane == 0 && b < kMsShifts) {
+        sm.lc[sg * kMsShifts + b] = c;
+        sm.log[2 * (sg * kMsShifts + b)] = sn;
       }
       __syncthreads();
-      // row operations: bulge b on rows (p, p+1), columns max(p-1, l) .. we
-      const int nact = bB - bA + 1;
-      for (int idx = tid; idx < nact * kMsW; idx += nthr) {
-        const int b = bA + idx / kMsW;
-        const int p = l + tt - 3 * b;
-        const int j = ((p == l) ? l : p - 1) + idx % kMsW;
-        if (j > we) continue;
-        const int k = p - sm.firstp[b];
-        const double c = sm.lc[b * kMsLog + k];
-        const cplx sn = sm.ls[b * kMsLog + k];
-        const cplx a = MSW(p - ws, j - ws), bb = MSW(p + 1 - ws, j - ws);
-        MSW(p - ws, j - ws) = cfma(sn, bb, cscale(a, c));
-        MSW(p + 1 - ws, j - ws) = cfma(cneg(cconj(sn)), a, cscale(bb, c));
+      if (on) {
+        // column operations: columns (p, p+1), rows ws .. min(p+2, i)
+        const int rn = min(p + 2, i) - ws;
+#pragma unroll
+        for (int q = 0; q < (kMsW + 31) / 32; ++q) {
+          const int r = lane + 32 * q;
+          if (r <= rn) {
+            const cplx a = MSW(r, p - ws), bb = MSW(r, p + 1 - ws);
+            MSW(r, p - ws) = cfma(cconj(sn), bb, cscale(a, c));
+            MSW(r, p + 1 - ws) = cfma(cneg(sn), a, cscale(bb, c));
+          }
+        }
       }
       __syncthreads();
-      if (tid >= bA && tid <= bB) {
-        const int p = l + tt - 3 * tid;
-        if (p > l) MSW(p + 1 - ws, p - 1 - ws) = mkc(0.0, 0.0);
-      }
-      // column operations: bulge b on columns (p, p+1), rows ws .. min(p+2, i)
-      for (int idx = tid; idx < nact * kMsW; idx += nthr) {
-        const int b = bA + idx / kMsW;
-        const int p = l + tt - 3 * b;
-        const int r = ws + idx % kMsW;
-        if (r > min(p + 2, i)) continue;
-        const int k = p - sm.firstp[b];
-        const double c = sm.lc[b * kMsLog + k];
-        const cplx sn = sm.ls[b * kMsLog + k];
-        const cplx a = MSW(r - ws, p - ws), bb = MSW(r - ws, p + 1 - ws);
-        MSW(r - ws, p - ws) = cfma(cconj(sn), bb, cscale(a, c));
-        MSW(r - ws, p + 1 - ws) = cfma(cneg(sn), a, cscale(bb, c));
-      }
-      __syncthreads();
+    }
+    // identity steps up to a whole replay group
+    const int npad = (nsteps + kMsPre - 1) / kMsPre * kMsPre;
+    for (int idx = nsteps * kMsShifts + tid; idx < npad * kMsShifts; idx += nthr) {
+      sm.lc[idx] = 1.0;
+      sm.log[2 * idx] = mkc(0.0, 0.0);
     }
 #ifdef RCWA_EIG_STATS
     const long long c_mid = clock64();
@@ -1259,41 +1484,14 @@ __device__ void ms_sweep(cplx* T, int ldt, cplx* Z, int n, int l, int i, int s, 
 #endif
     if (tm.rank == 0)
       for (int idx = tid; idx < w * w; idx += nthr) T[(size_t)(ws + idx / w) * ldt + ws + idx % w] = MSW(idx / w, idx % w);
-    // rows/columns touched in this pass
-    int rlo = i + 1, rhi = -1;
-    for (int b = 0; b < s; ++b)
-      if (sm.cnt[b] > 0) { rlo = min(rlo, sm.firstp[b]); rhi = max(rhi, sm.firstp[b] + sm.cnt[b]); }
-    const int nsteps = t1 - t;
-    // replay table per chain step and bulge: the log slot of the bulge's
-    // rotation at that step (the identity slot while it is inactive), so the
-    // chains interleave without branches
-    for (int idx = tid; idx < nsteps * kMsShifts; idx += nthr) {
-      const int sg = idx / kMsShifts, b = idx % kMsShifts;
-      int slot = kMsW;
-      if (b < s) {
-        const int k = sg - sm.tfirst[b];
-        if (k >= 0 && k < sm.cnt[b]) slot = k;
-      }
-      sm.ix[idx] = slot;
-    }
     __syncthreads();
     const int top0 = l + t - 3 * (kMsShifts - 1);
-    const int nR = (n - 1 - we + 31) / 32, nU = (ws + 31) / 32, nZ = (n + 31) / 32;
-    for (int task = warp + nwarp * tm.rank; task < nR + nU + nZ; task += nwarp * tm.size) {
-      if (task < nR) {
-        // T(rlo..rhi, j), j right of the window: row rotations, lane = column
-        const int j = we + 1 + 32 * task + lane;
-        if (j < n) replay_frame<true>(T + j, (size_t)ldt, top0, nsteps, rlo, rhi, sm);
-      } else if (task < nR + nU) {
-        // T(r, rlo..rhi), r above the window: column rotations, lane = row
-        const int r = 32 * (task - nR) + lane;
-        if (r < ws) replay_frame<false>(T + (size_t)r * ldt, (size_t)1, top0, nsteps, rlo, rhi, sm);
-      } else {
-        // Z(r, rlo..rhi) (column-major): column rotations, lane = row
-        const int r = 32 * (task - nR - nU) + lane;
-        if (r < n) replay_frame<false>(Z + r, (size_t)n, top0, nsteps, rlo, rhi, sm);
-      }
-    }
+    const bool scaled = replay_coefficients(sm, top0, ws, npad);
+    __syncthreads();
+    // indices touched in this pass
+    const int rlo = max(l, l + t - 3 * (s - 1)), rhi = min(i, l + t1);
+    if (scaled) replay_lines<true>(T, ldt, Z, n, ws, we, top0, npad, rlo, rhi, tm);
+    else replay_lines<false>(T, ldt, Z, n, ws, we, top0, npad, rlo, rhi, tm);
     tm.sync();
 #ifdef RCWA_EIG_STATS
     STAT_ADD(4, clock64() - c_mid);
@@ -1302,14 +1500,15 @@ __device__ void ms_sweep(cplx* T, int ldt, cplx* Z, int n, int l, int i, int s, 
   }
 }
 
-// Schur form by multishift sweeps on active blocks of at least ms_min rows
-// (ms_min >= kMsMin) and single-shift sweeps on smaller ones.  Returns 0 or
+// Schur form by early deflation and multishift sweeps; an active block that
+// fits the early-deflation window is finished there, in shared memory (single
+// shifts take over if the window's iteration runs out).  Returns 0 or
 // RCWA_ERR_NOCONV.  With a team of several CTAs the first CTA finds each
 // split point and runs the single-shift sweeps, and every decision that
 // steers the team's barriers comes from the first CTA through ctrl (global
 // scratch of at least 8 ints), so all CTAs take the same path.
-__device__ int schur_ms(cplx* T, int ldt, cplx* Z, int n, int ms_min, const MsSmem& sm, int sweep_cap,
-                        const Team& tm, int* ctrl) {
+__device__ int schur_ms(cplx* T, int ldt, cplx* Z, int n, const MsSmem& sm, int sweep_cap, const Team& tm,
+                        int* ctrl) {
   const double ulp = 2.0 * RCWA_DBL_EPS;
   const double smlnum = RCWA_DBL_MIN * ((double)n / ulp);
   const int tid = threadIdx.x;
@@ -1341,9 +1540,28 @@ __device__ int schur_ms(cplx* T, int ldt, cplx* Z, int n, int ms_min, const MsSm
     last_i = i;
     last_l = l;
     const int m = i - l + 1;
-    if (m < ms_min) {
-      // small blocks: single-shift sweeps whose off-window updates stream
-      // only the rotated pairs (cheaper than full tiles for few rotations)
+    // aggressive early deflation on the trailing window; its undeflated
+    // eigenvalues are the next sweep's shifts
+    int s = kMsShifts, cnt = 0;
+    bool have_shifts = false;
+#ifdef RCWA_EIG_STATS
+    const long long c_aed = clock64();
+#endif
+    const int nd = aed(T, ldt, Z, n, l, i, sm, tm, ctrl, &cnt);
+#ifdef RCWA_EIG_STATS
+    STAT_ADD(8, clock64() - c_aed);
+    STAT_ADD(11, 1);
+    STAT_ADD(12, nd > 0 ? nd : 0);
+#endif
+    if (nd > 0) {
+      stall = 0;
+      i -= nd;
+      if (100 * nd > kAedNibble * kAedW || i - l < kAedW) {
+        if (++sweeps > budget) return RCWA_ERR_NOCONV;
+        continue;
+      }
+    } else if (m <= kAedW) {
+      // the window's iteration ran out: a single-shift sweep
       cplx shift;
       if (stall == 10 || stall == 30)
         shift = cadd(T[(size_t)l * ldt + l], mkc(0.75 * cabs1(T[(size_t)(l + 1) * ldt + l]), 0.0));
@@ -1354,50 +1572,20 @@ __device__ int schur_ms(cplx* T, int ldt, cplx* Z, int n, int ms_min, const MsSm
                                 T[(size_t)i * ldt + i - 1], T[(size_t)i * ldt + i]);
       __syncthreads();
       STAT_ADD(1, 1);
-#ifdef RCWA_EIG_STATS
-      const long long c_ss = clock64();
-#endif
-      if (lead) qr_sweep(T, ldt, Z, n, l, i, shift, reinterpret_cast<cplx(*)[kWin + 1]>(sm.Wt), sm.lc, sm.ls);
-#ifdef RCWA_EIG_STATS
-      STAT_ADD(9, clock64() - c_ss);
-#endif
+      if (lead) qr_sweep(T, ldt, Z, n, l, i, shift, reinterpret_cast<cplx(*)[kWin + 1]>(sm.Wt), sm.lc, sm.log);
       if (++sweeps > budget) return RCWA_ERR_NOCONV;
       continue;
     }
-    // aggressive early deflation on the trailing window; its undeflated
-    // eigenvalues are the next sweep's shifts
-    int s = kMsShifts, ib = i;
-    bool have_shifts = false;
-    {
-#ifdef RCWA_EIG_STATS
-      const long long c_aed = clock64();
-#endif
-      int cnt = 0;
-      const int nd = aed(T, ldt, Z, n, l, i, sm, tm, ctrl, &cnt);
-#ifdef RCWA_EIG_STATS
-      STAT_ADD(8, clock64() - c_aed);
-      STAT_ADD(11, 1);
-      STAT_ADD(12, nd > 0 ? nd : 0);
-#endif
-      if (nd > 0) {
-        stall = 0;
-        if (100 * nd > kAedNibble * kAedW || i - nd - l + 1 < ms_min) {
-          if (++sweeps > budget) return RCWA_ERR_NOCONV;
-          continue;
-        }
-        ib = i - nd;
-      }
-      if (nd >= 0 && cnt >= kMsShifts / 2) {
-        s = cnt;
-        have_shifts = true;
-      }
+    if (nd >= 0 && cnt >= kMsShifts / 2) {
+      s = cnt;
+      have_shifts = true;
     }
     __syncthreads();
     {
       STAT_ADD(0, 1);
       if (tid < 32) {
         cplx* B = sm.work;  // s x s, stride s + 1
-        const int o = ib - s + 1;
+        const int o = i - s + 1;
         if (stall > 0 && stall % 6 == 0) {
           for (int k = tid; k < s; k += 32)
             sm.shifts[k] = cadd(T[(size_t)(o + k) * ldt + o + k],
@@ -1411,7 +1599,7 @@ __device__ int schur_ms(cplx* T, int ldt, cplx* Z, int n, int ms_min, const MsSm
       }
     }
     __syncthreads();
-    ms_sweep(T, ldt, Z, n, l, ib, s, sm, tm);
+    ms_sweep(T, ldt, Z, n, l, i, s, sm, tm);
     if (++sweeps > budget) return RCWA_ERR_NOCONV;
   }
   return 0;
@@ -1433,15 +1621,8 @@ __device__ bool hessenberg_finite(const cplx* T, int ldt, int n, int* redi) {
 }
 
 __global__ void __launch_bounds__(kMsThreads) schur_ms_kernel(cplx* const* Aarr, int n, int lda, cplx* w_all,
-                                                             void* work, int* info_all, int ms_min, int sweep_cap) {
-  extern __shared__ __align__(16) unsigned char dsm[];
-  const MsSmem sm = carve_ms_smem(dsm);
-  // identity slot of every bulge's rotation log (inactive chain steps)
-  for (int b = threadIdx.x; b < kMsShifts; b += blockDim.x) {
-    sm.lc[b * kMsLog + kMsW] = 1.0;
-    sm.ls[b * kMsLog + kMsW] = mkc(0.0, 0.0);
-  }
-  __syncthreads();
+                                                             void* work, int* info_all, int sweep_cap) {
+  const MsSmem sm = carve_ms_smem(ms_dsm);
   // one matrix per team (cluster) of CTAs
   const Team tm = cluster_team();
   const int mb = blockIdx.x / tm.size;
@@ -1462,11 +1643,20 @@ __global__ void __launch_bounds__(kMsThreads) schur_ms_kernel(cplx* const* Aarr,
     tm.sync();
     fin = __ldcg(ctrl + 5) != 0;
   }
-  const int status = fin ? schur_ms(A, lda, s.Z, n, ms_min, sm, sweep_cap, tm, ctrl) : RCWA_ERR_NONFINITE;
+  const int status = fin ? schur_ms(A, lda, s.Z, n, sm, sweep_cap, tm, ctrl) : RCWA_ERR_NONFINITE;
 #ifdef RCWA_EIG_STATS
   STAT_ADD(10, clock64() - c_schur);
 #endif
   if (tm.rank == 0) {
+    const double f = s.scale[0];
+    if (f != 1.0) {
+      __syncthreads();
+      for (size_t idx = threadIdx.x; idx < (size_t)n * n; idx += blockDim.x) {
+        cplx* const v = A + (idx / n) * lda + idx % n;
+        *v = cscale(*v, f);
+      }
+      __syncthreads();
+    }
     cplx* w = w_all + (size_t)mb * n;
     for (int k = threadIdx.x; k < n; k += blockDim.x) w[k] = A[(size_t)k * lda + k];
     if (threadIdx.x == 0) info_all[mb] = status;
@@ -1560,24 +1750,63 @@ constexpr int kHessThreads = 512;
 template <bool kTeam>
 __global__ void __launch_bounds__(kHessThreads) hessenberg_kernel(cplx* const* Aarr, int n, int lda, void* work) {
   __shared__ double red[kHessThreads / 32];
+  __shared__ int redi[kHessThreads / 32];
   __shared__ TileSmem tsm;
   // one matrix per team (cluster) of CTAs
   const Team tm = kTeam ? cluster_team() : Team{0, 1};
   const int mb = blockIdx.x / tm.size;
   const Scratch s = scratch_for(work, n, mb);
-  hessenberg_blocked<kTeam>(Aarr[mb], n, lda, s, red, tsm, tm);
+  cplx* A = Aarr[mb];
+  // a matrix whose products could leave the normal range is reduced and
+  // iterated at a power of two of its size (exact); the Schur kernel scales
+  // its result back
+  int ex = 0;
+  for (int i = threadIdx.x >> 5; i < n; i += blockDim.x >> 5) {
+    int e4 = 0;
+#pragma unroll 4
+    for (int j = threadIdx.x & 31; j < n; j += 32) {
+      const cplx v = A[(size_t)i * lda + j];
+      e4 = max(e4, max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff));
+    }
+    ex = max(ex, e4 >> 20);
+  }
+  ex = block_max_int(ex, redi) - 1023;
+  const int sh = ex > 100 ? min(ex, 1000) : ex < -100 ? max(ex, -1000) : 0;
+  if (sh != 0) {
+    const double f = scalbn(1.0, -sh);
+    const int per = (n + tm.size - 1) / tm.size;
+    tm.sync();  // every CTA has read the matrix
+    for (int i = tm.rank * per; i < min(n, (tm.rank + 1) * per); ++i)
+      for (int j = threadIdx.x; j < n; j += blockDim.x) A[(size_t)i * lda + j] = cscale(A[(size_t)i * lda + j], f);
+    tm.sync();
+  }
+  if (tm.rank == 0 && threadIdx.x == 0) s.scale[0] = scalbn(1.0, sh);
+  hessenberg_blocked<kTeam>(A, n, lda, s, red, tsm, tm);
 }
 
-__global__ void __launch_bounds__(kEigThreads) schur_kernel(cplx* const* Aarr, int n, int lda, cplx* w_all,
-                                                           void* work, int* info_all, int sweep_cap) {
-  __shared__ cplx Wt[kWin][kWin + 1];
-  __shared__ int redi[kEigThreads / 32];
-  __shared__ double rc[kWin];
-  __shared__ cplx rs[kWin];
+template <int Q>
+__global__ void __launch_bounds__(kBlkThreads) schur_block_kernel(cplx* const* Aarr, int n, int lda, cplx* w_all,
+                                                                 void* work, int* info_all, int sweep_cap) {
+  extern __shared__ __align__(16) unsigned char blk_dsm[];
+  __shared__ int redi[kBlkThreads / 32];
   cplx* A = Aarr[blockIdx.x];
+  cplx* T = reinterpret_cast<cplx*>(blk_dsm);
   const Scratch s = scratch_for(work, n, blockIdx.x);
-  const int status = hessenberg_finite(A, lda, n, redi) ? schur(A, lda, s.Z, n, Wt, rc, rs, redi, sweep_cap)
-                                                       : RCWA_ERR_NONFINITE;
+  const int ld = blk_ld(n);
+  int status = RCWA_ERR_NONFINITE;
+  if (hessenberg_finite(A, lda, n, redi)) {
+    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
+      const int r = idx / n, c = idx % n;
+      T[r * ld + c] = r <= c + 1 ? A[(size_t)r * lda + c] : mkc(0.0, 0.0);
+    }
+    __syncthreads();
+    status = schur_block<Q>(T, ld, s.Z, n, sweep_cap);
+    __syncthreads();
+    const double f = s.scale[0];
+    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x)
+      A[(size_t)(idx / n) * lda + idx % n] = cscale(T[(idx / n) * ld + idx % n], f);
+    __syncthreads();
+  }
   cplx* w = w_all + (size_t)blockIdx.x * n;
   for (int k = threadIdx.x; k < n; k += blockDim.x) w[k] = A[(size_t)k * lda + k];
   if (threadIdx.x == 0) info_all[blockIdx.x] = status;
@@ -1615,8 +1844,8 @@ std::atomic<int> g_qr_sweep_cap{0};
 // automatic choice), set by rcwa_set_eig_cluster.
 std::atomic<int> g_eig_team{0};
 
-// Matrices of at least this order use a team of CTAs when the batch leaves
-// SMs idle.
+// rcwa_eig_cluster_size reports the automatic team of orders from here on
+// (smaller ones report 1; their launches choose by the same rule).
 constexpr int kTeamMinN = 1024;
 
 // Clusters of `size` CTAs of `kernel` that fit on the device at once.
@@ -1641,30 +1870,30 @@ int active_clusters(K kernel, int threads, size_t smem, int size) {
   return nc;
 }
 
-// Team size for a batch of order-n matrices: the largest (up to 8) whose
-// clusters of both kernels all fit on the device in one wave, when the batch
-// alone would leave at least half of the SMs idle; 1 otherwise.
-int eig_team_size(int n, int batch, int ms_smem) {
-  const int forced = g_eig_team.load();
-  if (forced > 0) return forced;
-  if (n < kTeamMinN) return 1;
+// Team size for a batch of order-n matrices: the largest (up to 8, and a CTA
+// per 64 rows) whose clusters of both kernels all fit on the device in one
+// wave, when the batch alone would leave at least half of the SMs idle; 1
+// otherwise.
+int eig_team_auto(int n, int batch) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (2 * batch > sms) return 1;
+  if (batch <= 0 || 2 * batch > sms) return 1;
+  const int most = std::min(std::min(8, sms / batch), std::max(1, n / 64));
   static std::mutex mu;
-  static std::map<std::pair<int, int>, int> cache;  // (device, batch) -> size
+  static std::map<std::tuple<int, int, int>, int> cache;  // (device, batch, largest size) -> size
   std::lock_guard<std::mutex> lk(mu);
-  auto it = cache.find({dev, batch});
+  const auto key = std::make_tuple(dev, batch, most);
+  auto it = cache.find(key);
   if (it != cache.end()) return it->second;
   int pick = 1;
-  for (int c = std::min(8, sms / batch); c >= 2; --c)
+  for (int c = most; c >= 2; --c)
     if (active_clusters(hessenberg_kernel<true>, kHessThreads, 0, c) >= batch &&
-        active_clusters(schur_ms_kernel, kMsThreads, (size_t)ms_smem, c) >= batch) {
+        active_clusters(schur_ms_kernel, kMsThreads, kMsSmemBytes, c) >= batch) {
       pick = c;
       break;
     }
-  cache[{dev, batch}] = pick;
+  cache[key] = pick;
   return pick;
 }
 
@@ -1689,6 +1918,17 @@ cudaError_t launch_team(K kernel, int batch, int team, int threads, size_t smem,
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
+
+template <int Q>
+cudaError_t launch_block(cplx* const* A, int n, int lda, cplx* w, void* work, int* info, int sweep_cap, int batch,
+                         cudaStream_t st) {
+  static SmemAttrOnce attr;
+  const cudaError_t e = attr.ensure(schur_block_kernel<Q>, (int)blk_smem(std::min(32 * Q, kBlkMax)));
+  if (e != cudaSuccess) return e;
+  schur_block_kernel<Q><<<batch, kBlkThreads, blk_smem(n), st>>>(A, n, lda, w, work, info, sweep_cap);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 extern "C" int rcwa_set_qr_sweep_limit(int sweeps) {
@@ -1705,13 +1945,15 @@ extern "C" int rcwa_set_eig_cluster(int ctas) {
 
 extern "C" int rcwa_eig_cluster_size(int n, int batch) {
   if (n < kMsMin || batch <= 0) return 1;
-  return eig_team_size(n, batch, (int)kMsSmemBytes);
+  const int forced = g_eig_team.load();
+  if (forced > 0) return forced;
+  return n < kTeamMinN ? 1 : eig_team_auto(n, batch);
 }
 
 cudaError_t zgeev_batched(cplx* const* A, int n, int lda, cplx* w, cplx* const* VR, int ldv, void* work,
                           int* info, int batch, cudaStream_t st, StageProf* prof, int ms_min) {
   if (batch <= 0 || n <= 0) return cudaSuccess;
-  ms_min = max(ms_min, kMsMin);
+  ms_min = ms_min <= 0 ? kBlkMax + 1 : max(ms_min, kMsMin);
   const int sweep_cap = g_qr_sweep_cap.load();
   StageProf none;
   StageProf& P = prof ? *prof : none;
@@ -1719,22 +1961,24 @@ cudaError_t zgeev_batched(cplx* const* A, int n, int lda, cplx* w, cplx* const* 
   cudaError_t e = attr.ensure(schur_ms_kernel, (int)kMsSmemBytes);
   if (e != cudaSuccess) return e;
   // a team of CTAs per matrix where the batch is too small to fill the GPU
-  // (the single-shift kernel for small orders always runs one CTA)
-  const int team = n < ms_min ? 1 : eig_team_size(n, batch, (int)kMsSmemBytes);
+  // (matrices held in shared memory always run one CTA)
+  const bool block = n < ms_min && n <= kBlkMax;
+  const int forced = g_eig_team.load();
+  const int team = block ? 1 : forced > 0 ? forced : eig_team_auto(n, batch);
   e = team > 1 ? launch_team(hessenberg_kernel<true>, batch, team, kHessThreads, 0, st, A, n, lda, work)
                : launch_team(hessenberg_kernel<false>, batch, 1, kHessThreads, 0, st, A, n, lda, work);
   if (e != cudaSuccess) return e;
   ++launch_counter();
   P.mark(st, kStHessenberg);
-  if (n < ms_min) {
-    schur_kernel<<<batch, kEigThreads, 0, st>>>(A, n, lda, w, work, info, sweep_cap);
-    ++launch_counter();
+  if (block) {
+    e = n <= 32 ? launch_block<1>(A, n, lda, w, work, info, sweep_cap, batch, st)
+        : n <= 64 ? launch_block<2>(A, n, lda, w, work, info, sweep_cap, batch, st)
+                  : launch_block<4>(A, n, lda, w, work, info, sweep_cap, batch, st);
   } else {
-    if ((e = launch_team(schur_ms_kernel, batch, team, kMsThreads, kMsSmemBytes, st, A, n, lda, w, work, info,
-                         ms_min, sweep_cap)) != cudaSuccess)
-      return e;
-    ++launch_counter();
+    e = launch_team(schur_ms_kernel, batch, team, kMsThreads, kMsSmemBytes, st, A, n, lda, w, work, info, sweep_cap);
   }
+  if (e != cudaSuccess) return e;
+  ++launch_counter();
   P.mark(st, kStSchur);
   trevc_kernel<<<batch, kEigThreads, 0, st>>>(A, n, lda, work);
   ++launch_counter();

@@ -122,8 +122,9 @@ int tune_candidates(int op, int n, int* out) {
 int tune_default_sms(int op, int n, int batch, int sms) {
   switch (op) {
     case kTuneLU: return zgetrf_default_schedule(n, batch, sms);
-    // whole matrices below 128 rows: the single-shift kernel (measured on
-    // B200: n = 98 in 61% of the multishift kernel's time; n = 242 slower)
+    // up to 116 rows: the kernel that holds the matrix in shared memory
+    // (measured on B200, block against multishift kernel: 303 x 82 6.3 / 13.6
+    // ms, 400 x 98 17.2 / 21.1 ms)
     case kTuneSchur: return (n >= kSchurCrossover && n < 128) ? 128 : kSchurCrossover;
     case kTuneProduct: return 0;
     default: return -1;

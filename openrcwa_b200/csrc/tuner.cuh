@@ -3,8 +3,9 @@
 // timed on this GPU.  Decisions:
 //   kTuneLU       LU factorisation schedule (0: one CTA per matrix, 1: panel
 //                 by panel over all SMs)
-//   kTuneSchur    Schur crossover: active blocks below it use single-shift
-//                 sweeps, larger ones multishift sweeps with early deflation
+//   kTuneSchur    Schur crossover: matrices below it (and of at most 116
+//                 rows) are iterated in shared memory, others by windowed
+//                 multishift sweeps with early deflation
 //   kTuneProduct  cascade products of mixed plans and their tile shape
 //                 (0: 3xTF32 on tcgen05, 128 x 128 tiles; 1: FP64 tensor path;
 //                 2: 3xTF32 on tcgen05, 128 x 256 tiles)
