@@ -229,9 +229,198 @@ __global__ void __launch_bounds__(kTileThreads) zgetrf_kernel(cplx* const* Aarr,
   if (tid == 0) info_all[b] = info;
 }
 
-// Panel width of the multi-launch LU, and the panel kernel's block size: a
-// whole SM per panel keeps enough loads in flight for the rank-1 updates,
-// whose rows come from L2.
+// ---- panel-by-panel LU ------------------------------------------------------
+// A panel is kRegW columns wide and lives in registers: one thread holds one
+// row's kRegW entries, so a rank-1 update is FP64 instructions only and the
+// panel crosses memory once.  Up to kRegT rows fit one CTA (128 registers a
+// thread); a taller panel is shared by a thread-block cluster of up to 8 CTAs
+// (n <= 4096), which exchange their pivot candidates and candidate rows
+// through distributed shared memory.  Bound by the latency of a column:
+// the warps' arg-max (three redux steps), two barriers, the reciprocal and the
+// update.  Whole factorisations (schedule 2) against 32-column panels updated
+// in L2, B200: 58 x 882 16.4 -> 8.9 ms, 46 x 494 5.3 -> 2.6 ms, 148 x 450 6.1 ->
+// 4.2 ms, 2 x 1250 12.1 -> 5.2 ms.  Same pivot rule and the same operations per entry as
+// lu_panel, so the panel's factors are the same for every cluster size.
+constexpr int kRegW = 16;
+constexpr int kRegT = 512;
+constexpr int kRegMaxRows = 8 * kRegT;
+
+// arg-max over a warp of (key, smallest row): keys are the bits of
+// non-negative doubles, which order like integers; NaN maps to 0, so that it
+// never wins against a number.  Every lane gets the result.
+__device__ __forceinline__ void warp_argmax(unsigned long long& key, int& row) {
+  const unsigned hi = (unsigned)(key >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+  row = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? row : 0x7fffffff);
+  key = ((unsigned long long)mh << 32) | ml;
+}
+
+__global__ void __launch_bounds__(kRegT) getrf_regpanel_kernel(cplx* const* Aarr, int n, int lda, int kb, int jb,
+                                                              int* ipiv_all, int* info_all) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  // slots alternate between columns, so that a column's values are overwritten
+  // only after a barrier that follows their last read
+  __shared__ unsigned long long s_key[2][kRegT / 32];
+  __shared__ int s_row[2][kRegT / 32];
+  __shared__ unsigned long long s_ckey[2];
+  __shared__ int s_crow[2];
+  __shared__ cplx s_cand[2][kRegW], s_jrow[2][kRegW];  // this CTA's candidate row; row j, in its owner's CTA
+  __shared__ cplx s_p[2][kRegW], s_j[2][kRegW];        // the pivot row and row j
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int tid = threadIdx.x, lane = tid & 31, nw = blockDim.x >> 5;
+  const int b = blockIdx.x / C;
+  cplx* A = Aarr[b];
+  int* ipiv = ipiv_all + (size_t)b * n;
+  int info = kb == 0 ? 0 : info_all[b];
+  const int i = kb + rank * (int)blockDim.x + tid;  // this thread's row
+  const bool in = i < n;
+  cplx a[kRegW];
+  cplx* const Ai = A + (size_t)i * lda + kb;
+#pragma unroll
+  for (int c = 0; c < kRegW; ++c) a[c] = in && c < jb ? Ai[c] : mkc(0.0, 0.0);
+#pragma unroll
+  for (int jj = 0; jj < kRegW; ++jj) {
+    if (jj >= jb) break;
+    const int j = kb + jj, bf = jj & 1;
+    const bool act = in && i >= j;
+    const double v = act ? cabs1(a[jj]) : 0.0;
+    unsigned long long key = v == v ? (unsigned long long)__double_as_longlong(v) : 0ull;
+    int row = act ? i : 0x7fffffff;
+    if (!act) key = 0ull;
+    warp_argmax(key, row);
+    if (lane == 0) { s_key[bf][tid >> 5] = key; s_row[bf][tid >> 5] = row; }
+    if (i == j) {
+#pragma unroll
+      for (int c = 0; c < kRegW; ++c) s_jrow[bf][c] = a[c];
+    }
+    __syncthreads();
+    key = lane < nw ? s_key[bf][lane] : 0ull;
+    row = lane < nw ? s_row[bf][lane] : 0x7fffffff;
+    warp_argmax(key, row);
+    const cplx *prow = s_cand[bf], *jrow = s_jrow[bf];
+    if (i == row) {
+#pragma unroll
+      for (int c = 0; c < kRegW; ++c) s_cand[bf][c] = a[c];
+    }
+    if (C > 1) {
+      if (tid == 0) { s_ckey[bf] = key; s_crow[bf] = row; }
+      cl.sync();
+      if (tid < 32) {
+        key = lane < C ? *cl.map_shared_rank(&s_ckey[bf], lane) : 0ull;
+        row = lane < C ? *cl.map_shared_rank(&s_crow[bf], lane) : 0x7fffffff;
+        warp_argmax(key, row);
+        // row >= j always: row j itself is a candidate
+        const int owner = (row - kb) / (int)blockDim.x, jowner = jj / (int)blockDim.x;
+        if (lane < kRegW) s_p[bf][lane] = *cl.map_shared_rank(&s_cand[bf][lane], owner);
+        else s_j[bf][lane - kRegW] = *cl.map_shared_rank(&s_jrow[bf][lane - kRegW], jowner);
+        if (lane == 0) s_crow[bf ^ 1] = row;  // read below, rewritten after the next column's barrier
+      }
+      prow = s_p[bf];
+      jrow = s_j[bf];
+    }
+    __syncthreads();
+    const int p = C > 1 ? s_crow[bf ^ 1] : row;
+    if (rank == 0 && tid == 0) ipiv[j] = p;
+    if (p != j) {
+      if (i == p) {
+#pragma unroll
+        for (int c = 0; c < kRegW; ++c) a[c] = jrow[c];
+      } else if (i == j) {
+#pragma unroll
+        for (int c = 0; c < kRegW; ++c) a[c] = prow[c];
+      }
+    }
+    const cplx piv = prow[jj];
+    cplx inv = mkc(1.0, 0.0);
+    if (piv.x == 0.0 && piv.y == 0.0) {
+      if (info == 0) info = j + 1;
+    } else {
+      inv = cdiv(mkc(1.0, 0.0), piv);
+    }
+    if (in && i > j) {
+      const cplx l = piv.x == 0.0 && piv.y == 0.0 ? a[jj] : cmul(a[jj], inv);
+      a[jj] = l;
+#pragma unroll
+      for (int c = jj + 1; c < kRegW; ++c) a[c] = cfma(cneg(l), prow[c], a[c]);
+    }
+  }
+  if (in) {
+#pragma unroll
+    for (int c = 0; c < kRegW; ++c)
+      if (c < jb) Ai[c] = a[c];
+  }
+  if (rank == 0 && tid == 0) info_all[b] = info;
+  // no CTA leaves while another may still read its candidate
+  if (C > 1) cl.sync();
+}
+
+// After a register panel: its row interchanges on every column outside the
+// panel, and U12 = L11^-1 A12 on the columns kb+jb .. ce-1.  One thread per
+// column: the interchanges are folded into one permutation of the (at most 2
+// kRegW) rows they touch, so that a column's loads are all in flight at once.
+__global__ void __launch_bounds__(128) getrf_swap_trsm_kernel(cplx* const* Aarr, int n, int lda, int kb, int jb, int ce,
+                                                              const int* ipiv_all) {
+  __shared__ int s_dst[2 * kRegW], s_src[2 * kRegW];
+  __shared__ cplx L[kRegW][kRegW + 1];
+  const int b = blockIdx.y, tid = threadIdx.x;
+  cplx* A = Aarr[b];
+  if (tid < 32) {
+    // lane q < kRegW: row kb + q; lane kRegW + q: the q-th pivot row, when it
+    // lies below the panel's own rows and no earlier lane has it
+    const int* ipiv = ipiv_all + (size_t)b * n + kb;
+    const int q0 = tid & (kRegW - 1);
+    const int p = q0 < jb ? ipiv[q0] : -1;
+    int at = tid < kRegW ? kb + tid : (p >= kb + kRegW ? p : -1);
+    for (int q = 0; q < kRegW - 1; ++q) {
+      const int o = __shfl_sync(0xffffffffu, at, kRegW + q);
+      if (tid > kRegW + q && at == o) at = -1;
+    }
+    int src = at;  // the row whose values end up at row `at`
+    for (int q = 0; q < jb; ++q) {
+      const int pq = __shfl_sync(0xffffffffu, p, q);
+      const unsigned m = __ballot_sync(0xffffffffu, at == pq);
+      const int lp = __ffs(m) - 1;
+      const int sq = __shfl_sync(0xffffffffu, src, q), sp = __shfl_sync(0xffffffffu, src, lp);
+      if (tid == q) src = sp;
+      if (tid == lp) src = sq;
+    }
+    s_dst[tid] = at == src ? -1 : at;
+    s_src[tid] = at == src ? -1 : src;
+  }
+  for (int idx = tid; idx < kRegW * kRegW; idx += blockDim.x) {
+    const int r = idx / kRegW, q = idx % kRegW;
+    L[r][q] = r < jb && q < r ? A[(size_t)(kb + r) * lda + kb + q] : mkc(0.0, 0.0);
+  }
+  __syncthreads();
+  int c = blockIdx.x * blockDim.x + tid;
+  if (c >= n - jb) return;
+  if (c >= kb) c += jb;  // the panel's own columns are already permuted
+  const bool solve = c >= kb && c < ce;
+  cplx x[2 * kRegW];
+#pragma unroll
+  for (int k = 0; k < 2 * kRegW; ++k) {
+    const int src = s_src[k];
+    if (src >= 0) x[k] = A[(size_t)src * lda + c];
+    else if (k < kRegW && k < jb && solve) x[k] = A[(size_t)(kb + k) * lda + c];
+  }
+  if (solve) {
+#pragma unroll
+    for (int r = 1; r < kRegW; ++r) {
+      if (r < jb)
+#pragma unroll
+        for (int q = 0; q < r; ++q) x[r] = cfma(cneg(L[r][q]), x[q], x[r]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 2 * kRegW; ++k) {
+    if (s_dst[k] >= 0) A[(size_t)s_dst[k] * lda + c] = x[k];
+    else if (k < kRegW && k > 0 && k < jb && solve) A[(size_t)(kb + k) * lda + c] = x[k];
+  }
+}
+
+// Matrices above kRegMaxRows rows: panels of kLuPanel columns updated in L2.  A
+// whole SM per panel keeps enough loads in flight for the rank-1 updates.
 constexpr int kLuPanel = 32;
 constexpr int kLuPanelThreads = 512;
 
@@ -682,6 +871,42 @@ cudaError_t launch_panel(cplx* const* A, int n, int lda, int kb, int jb, int* ip
 }
 }  // namespace
 
+namespace {
+// A register panel on the CTAs its rows need (or the forced cluster size).
+cudaError_t launch_regpanel(cplx* const* A, int n, int lda, int kb, int jb, int* ipiv, int* info, int batch,
+                            cudaStream_t st) {
+  const int rows = n - kb;
+  const int threads = rows <= 128 ? 128 : rows <= 256 ? 256 : kRegT;
+  const int team = std::max((rows + threads - 1) / threads, g_lu_team.load());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(batch * team);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = team;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, getrf_regpanel_kernel, A, n, lda, kb, jb, ipiv, info);
+}
+
+// A22 -= L21 U12 on the columns kb+jb .. ce-1
+cudaError_t panel_update(cplx* const* A, int n, int lda, int kb, int jb, int ce, int batch, cudaStream_t st) {
+  GemmArgs g{};
+  g.A = A; g.B = A; g.C = A; g.D = A;
+  g.offA = (size_t)(kb + jb) * lda + kb;
+  g.offB = (size_t)kb * lda + kb + jb;
+  g.offC = g.offD = (size_t)(kb + jb) * lda + kb + jb;
+  g.M = n - kb - jb; g.N = ce - kb - jb; g.K = jb;
+  g.lda = g.ldb = g.ldc = g.ldd = lda;
+  g.alpha = mkc(-1.0, 0.0); g.beta = mkc(1.0, 0.0); g.gammaI = mkc(0.0, 0.0);
+  g.batch = batch;
+  return zgemm_batched(g, st);
+}
+}  // namespace
+
 extern "C" int rcwa_set_lu_cluster(int ctas) {
   if (ctas < 0 || ctas > 8) return RCWA_ERR_INVALID;
   g_lu_team.store(ctas);
@@ -695,8 +920,8 @@ extern "C" int rcwa_lu_cluster_size(int n, int batch) {
 
 int zgetrf_default_schedule(int n, int batch, int sms) {
   if (sms <= 0) sms = sm_count();
-  // 128-column blocks from n = 256 on (measured on B200 at n = 882: 148
-  // matrices 41.9 -> 32.4 ms, 296 matrices 74.0 -> 57.5 ms against panel by panel)
+  // 128-column blocks from n = 256 on (measured on B200 against panel by panel:
+  // 58 x 882 13.6 -> 8.9 ms, 148 x 450 5.4 -> 4.2 ms; 2 x 1250 5.2 -> 6.2 ms)
   if (n <= 128 || batch >= 4 * sms) return 0;
   return n >= 256 ? 2 : 1;
 }
@@ -717,6 +942,20 @@ cudaError_t zgetrf_batched(cplx* const* A, int n, int lda, int* ipiv, int* info,
 cudaError_t zgetrf_columns(cplx* const* A, int n, int lda, int k0, int ce, int* ipiv, int* info, int batch,
                            cudaStream_t st) {
   if (batch <= 0 || k0 < 0 || ce > n || k0 >= ce) return cudaErrorInvalidValue;
+  if (n <= kRegMaxRows) {
+    for (int kb = k0; kb < ce; kb += kRegW) {
+      const int jb = min(kRegW, ce - kb);
+      cudaError_t e = launch_regpanel(A, n, lda, kb, jb, ipiv, info, batch, st);
+      if (e != cudaSuccess) return e;
+      ++launch_counter();
+      if (n == jb) break;  // nothing beside the panel
+      getrf_swap_trsm_kernel<<<dim3((n - jb + 127) / 128, batch), 128, 0, st>>>(A, n, lda, kb, jb, ce, ipiv);
+      ++launch_counter();
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+      if ((e = panel_update(A, n, lda, kb, jb, ce, batch, st)) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
   // a cluster of CTAs per matrix shares each panel when the batch leaves SMs idle
   const int team = lu_team_size(n, batch);
   for (int kb = k0; kb < ce; kb += kLuPanel) {
@@ -728,17 +967,7 @@ cudaError_t zgetrf_columns(cplx* const* A, int n, int lda, int k0, int ce, int* 
     if (m2 <= 0 || w <= 0) break;
     getrf_trsm_kernel<<<dim3((w + 63) / 64, batch), 64, 0, st>>>(A, lda, kb, jb, ce);
     ++launch_counter();
-    // A22 -= L21 U12 (the block's columns)
-    GemmArgs g{};
-    g.A = A; g.B = A; g.C = A; g.D = A;
-    g.offA = (size_t)(kb + jb) * lda + kb;
-    g.offB = (size_t)kb * lda + kb + jb;
-    g.offC = g.offD = (size_t)(kb + jb) * lda + kb + jb;
-    g.M = m2; g.N = w; g.K = jb;
-    g.lda = g.ldb = g.ldc = g.ldd = lda;
-    g.alpha = mkc(-1.0, 0.0); g.beta = mkc(1.0, 0.0); g.gammaI = mkc(0.0, 0.0);
-    g.batch = batch;
-    cudaError_t err = zgemm_batched(g, st);
+    const cudaError_t err = panel_update(A, n, lda, kb, jb, ce, batch, st);
     if (err != cudaSuccess) return err;
   }
   return cudaGetLastError();
