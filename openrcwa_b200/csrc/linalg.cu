@@ -355,6 +355,77 @@ __global__ void __launch_bounds__(kRegT) getrf_regpanel_kernel(cplx* const* Aarr
   if (C > 1) cl.sync();
 }
 
+// Matrices of at most kSmallLuMax rows: the whole matrix in shared memory, one
+// CTA each, right-looking column by column.  Every warp finds the pivot itself
+// (the same data, no exchange), so a column costs two barriers; bound by their
+// latency and the reciprocal.  Same pivot rule as lu_panel.
+// B200, against lu_panel in global memory: 400 x 98 2.27 -> 0.98 ms, 303 x 82
+// 1.64 -> 0.49 ms, one 50-row matrix 0.15 -> 0.06 ms.
+constexpr int kSmallLuMax = 116;
+constexpr int kSmallLuThreads = 256;
+__host__ __device__ constexpr size_t small_lu_smem(int n) { return sizeof(cplx) * (size_t)n * (n | 1); }
+
+__global__ void __launch_bounds__(kSmallLuThreads) getrf_small_kernel(cplx* const* Aarr, int n, int lda, int* ipiv_all,
+                                                                     int* info_all) {
+  extern __shared__ __align__(16) unsigned char small_smem[];
+  constexpr int Q = (kSmallLuMax + 31) / 32;
+  cplx* const S = reinterpret_cast<cplx*>(small_smem);
+  const int ld = n | 1, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kSmallLuThreads / 32;
+  cplx* const A = Aarr[blockIdx.x];
+  int* const ipiv = ipiv_all + (size_t)blockIdx.x * n;
+  int info = 0;
+  for (int idx = tid; idx < n * n; idx += kSmallLuThreads) S[(idx / n) * ld + idx % n] = A[(size_t)(idx / n) * lda + idx % n];
+  __syncthreads();
+  for (int j = 0; j < n; ++j) {
+    unsigned long long key = 0ull;
+    int row = 0x7fffffff;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int i = j + lane + 32 * q;
+      if (i < n) {
+        const double v = cabs1(S[i * ld + j]);
+        const unsigned long long k = v == v ? (unsigned long long)__double_as_longlong(v) : 0ull;
+        if (k > key || row == 0x7fffffff) { key = k; row = i; }
+      }
+    }
+    warp_argmax(key, row);
+    const int p = row;
+    if (tid == 0) ipiv[j] = p;
+    __syncthreads();  // every warp has read the column
+    if (p != j)
+      for (int c = tid; c < n; c += kSmallLuThreads) {
+        const cplx t = S[j * ld + c];
+        S[j * ld + c] = S[p * ld + c];
+        S[p * ld + c] = t;
+      }
+    __syncthreads();
+    const cplx piv = S[j * ld + j];
+    const bool zero = piv.x == 0.0 && piv.y == 0.0;
+    if (zero && info == 0) info = j + 1;
+    const cplx inv = zero ? mkc(1.0, 0.0) : cdiv(mkc(1.0, 0.0), piv);
+    cplx pr[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int c = j + 1 + lane + 32 * q;
+      pr[q] = c < n ? S[j * ld + c] : mkc(0.0, 0.0);
+    }
+#pragma unroll 2
+    for (int i = j + 1 + warp; i < n; i += nw) {
+      const cplx l = cmul(S[i * ld + j], inv);
+      __syncwarp();
+      if (lane == 0) S[i * ld + j] = l;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int c = j + 1 + lane + 32 * q;
+        if (c < n) S[i * ld + c] = cfma(cneg(l), pr[q], S[i * ld + c]);
+      }
+    }
+    __syncthreads();
+  }
+  for (int idx = tid; idx < n * n; idx += kSmallLuThreads) A[(size_t)(idx / n) * lda + idx % n] = S[(idx / n) * ld + idx % n];
+  if (tid == 0) info_all[blockIdx.x] = info;
+}
+
 // After a register panel: its row interchanges on every column outside the
 // panel, and U12 = L11^-1 A12 on the columns kb+jb .. ce-1.  One thread per
 // column: the interchanges are folded into one permutation of the (at most 2
@@ -930,6 +1001,14 @@ cudaError_t zgetrf_batched(cplx* const* A, int n, int lda, int* ipiv, int* info,
                            cudaStream_t st, int schedule) {
   if (batch <= 0 || n <= 0) return cudaSuccess;
   if (schedule < 0) schedule = zgetrf_default_schedule(n, batch);
+  if (schedule == 0 && n <= kSmallLuMax) {
+    static SmemAttrOnce attr;
+    const cudaError_t e = attr.ensure(getrf_small_kernel, (int)small_lu_smem(kSmallLuMax));
+    if (e != cudaSuccess) return e;
+    getrf_small_kernel<<<batch, kSmallLuThreads, small_lu_smem(n), st>>>(A, n, lda, ipiv, info);
+    ++launch_counter();
+    return cudaGetLastError();
+  }
   if (schedule == 0) {
     zgetrf_kernel<<<batch, kTileThreads, 0, st>>>(A, n, lda, ipiv, info);
     ++launch_counter();
@@ -973,18 +1052,19 @@ cudaError_t zgetrf_columns(cplx* const* A, int n, int lda, int k0, int ce, int* 
   return cudaGetLastError();
 }
 
-// From this order on, solves with at least 64 right-hand sides run blocked
-// (lu_blocked.cu: 128-row triangles plus batched GEMM updates over the whole
-// grid) instead of one CTA per 64-column slab; a build parameter.
-#ifndef RCWA_BLOCKED_SOLVE_MIN_N
-#define RCWA_BLOCKED_SOLVE_MIN_N 256
-#endif
-constexpr int kBlockedSolveMinN = RCWA_BLOCKED_SOLVE_MIN_N;
+// From this order and this many right-hand sides on, solves run blocked
+// (lu_blocked.cu: 128-row triangles with a thread per right-hand side and the
+// entries of 32 rows in registers, plus batched GEMM updates over the whole
+// grid) instead of one CTA per 64-column slab, whose triangles wait for a
+// dependent load per entry (B200, interface solves of 600 x 58 1.43 -> 0.63 ms,
+// 400 x 98 3.32 -> 1.75 ms, 200 x 198 7.05 -> 2.76 ms).  Below 16 a quarter's
+// 32 rows are mostly padding.
+constexpr int kBlockedSolveMin = 16;
 
 cudaError_t zgetrs_batched(const cplx* const* LU, int n, int lda, const int* ipiv, cplx* const* B,
                            int nrhs, int ldb, int batch, cudaStream_t st) {
   if (batch <= 0 || n <= 0 || nrhs <= 0) return cudaSuccess;
-  if (n >= kBlockedSolveMinN && nrhs >= 64)
+  if (n >= kBlockedSolveMin && nrhs >= kBlockedSolveMin)
     return zgetrs_blocked_batched(LU, n, lda, ipiv, B, nrhs, ldb, batch, false, nullptr, st);
   dim3 grid((nrhs + 63) / 64, batch);
   zgetrs_kernel<false><<<grid, kTileThreads, 0, st>>>(LU, n, lda, ipiv, B, nrhs, ldb);
@@ -995,7 +1075,7 @@ cudaError_t zgetrs_batched(const cplx* const* LU, int n, int lda, const int* ipi
 cudaError_t zgetri_batched(const cplx* const* LU, int n, int lda, const int* ipiv, cplx* const* X, int ldx,
                            int batch, cudaStream_t st) {
   if (batch <= 0 || n <= 0) return cudaSuccess;
-  if (n >= kBlockedSolveMinN) return zgetrs_blocked_batched(LU, n, lda, ipiv, X, n, ldx, batch, true, nullptr, st);
+  if (n >= kBlockedSolveMin) return zgetrs_blocked_batched(LU, n, lda, ipiv, X, n, ldx, batch, true, nullptr, st);
   dim3 grid((n + 63) / 64, batch);
   zgetrs_kernel<true><<<grid, kTileThreads, 0, st>>>(LU, n, lda, ipiv, X, n, ldx);
   ++launch_counter();

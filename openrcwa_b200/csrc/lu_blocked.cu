@@ -61,14 +61,14 @@ __device__ __forceinline__ void load_tile32(cplx (*Tsm)[33], const cplx* LU, int
 // T of LU at (r0, r0): unit lower (forward) or upper (backward); columns
 // [c_lo, nrhs) only (the inverse's forward pass skips columns whose rows
 // here are still zero).
-template <bool kUpper>
-__global__ void __launch_bounds__(kDiagThreads) trsm_diag_kernel(const cplx* const* LUarr, int lda,
+template <bool kUpper, int kThreads>
+__global__ void __launch_bounds__(kThreads) trsm_diag_kernel(const cplx* const* LUarr, int lda,
                                                                  cplx* const* Barr, int ldb, int nrhs, int r0,
                                                                  int rows, int c_lo) {
   __shared__ cplx Tsm[32][33];
   __shared__ cplx dinv[32];  // backward: reciprocals of the quarter's diagonal
   const int b = blockIdx.y;
-  const int c = c_lo + blockIdx.x * kDiagThreads + threadIdx.x;
+  const int c = c_lo + blockIdx.x * kThreads + threadIdx.x;
   const bool col = c < nrhs;
   const cplx* LU = LUarr[b];
   cplx* B = Barr[b];
@@ -133,6 +133,21 @@ __global__ void __launch_bounds__(kDiagThreads) trsm_diag_kernel(const cplx* con
   }
 }
 
+// Launch over the columns [c_lo, nrhs): kDiagThreads right-hand sides per CTA,
+// or 64 where that leaves SMs without one.
+template <bool kUpper>
+cudaError_t trsm_diag(const cplx* const* LU, int lda, cplx* const* B, int ldb, int nrhs, int r0, int rows, int c_lo,
+                      int batch, cudaStream_t st) {
+  const int cols = nrhs - c_lo;
+  if (cols > 128)
+    trsm_diag_kernel<kUpper, kDiagThreads><<<dim3((cols + kDiagThreads - 1) / kDiagThreads, batch), kDiagThreads, 0,
+                                             st>>>(LU, lda, B, ldb, nrhs, r0, rows, c_lo);
+  else
+    trsm_diag_kernel<kUpper, 64><<<dim3((cols + 63) / 64, batch), 64, 0, st>>>(LU, lda, B, ldb, nrhs, r0, rows, c_lo);
+  ++launch_counter();
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 namespace {
@@ -151,10 +166,8 @@ cudaError_t zgetrf_blocked_batched(cplx* const* A, int n, int lda, int* ipiv, in
     if ((e = zgetrf_columns(A, n, lda, kb, ke, ipiv, info, batch, st)) != cudaSuccess) return e;
     if (ke == n) break;
     // U12 = L11^-1 A12: the block's rows, columns ke .. n-1
-    trsm_diag_kernel<false><<<dim3((n - ke + kDiagThreads - 1) / kDiagThreads, batch), kDiagThreads, 0, st>>>(
-        (const cplx* const*)A, lda, A, lda, n, kb, ke - kb, ke);
-    ++launch_counter();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = trsm_diag<false>((const cplx* const*)A, lda, A, lda, n, kb, ke - kb, ke, batch, st)) != cudaSuccess)
+      return e;
     // A22 -= L21 U12
     GemmArgs g{};
     g.A = (const cplx* const*)A; g.offA = (size_t)ke * lda + kb;
@@ -188,10 +201,7 @@ cudaError_t zgetrs_blocked_batched(const cplx* const* LU, int n, int lda, const 
     const int rw = min(kNb, n - kb);
     // the inverse's rows kb.. are zero in the columns past the block (L^-1 is lower triangular)
     const int c_lo = 0, c_hi = inverse ? kb + rw : nrhs;
-    trsm_diag_kernel<false><<<dim3((c_hi - c_lo + kDiagThreads - 1) / kDiagThreads, batch), kDiagThreads, 0, st>>>(
-        LU, lda, B, ldb, c_hi, kb, rw, c_lo);
-    ++launch_counter();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = trsm_diag<false>(LU, lda, B, ldb, c_hi, kb, rw, c_lo, batch, st)) != cudaSuccess) return e;
     const int m2 = n - kb - rw;
     if (m2 > 0) {
       GemmArgs g{};
@@ -209,10 +219,7 @@ cudaError_t zgetrs_blocked_batched(const cplx* const* LU, int n, int lda, const 
   // backward: U
   for (int kb = ((n - 1) / kNb) * kNb; kb >= 0; kb -= kNb) {
     const int rw = min(kNb, n - kb);
-    trsm_diag_kernel<true><<<dim3((nrhs + kDiagThreads - 1) / kDiagThreads, batch), kDiagThreads, 0, st>>>(
-        LU, lda, B, ldb, nrhs, kb, rw, 0);
-    ++launch_counter();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = trsm_diag<true>(LU, lda, B, ldb, nrhs, kb, rw, 0, batch, st)) != cudaSuccess) return e;
     if (kb > 0) {
       GemmArgs g{};
       g.A = LU; g.offA = (size_t)kb;

@@ -1,5 +1,6 @@
-"""The register-panel LU at its edges (16-column panels, 128-column blocks, one
-to several CTAs per panel), through the star product's inverse, on matrices
+"""The LU and the solves at their edges (the shared-memory kernel up to 116 rows;
+16-column register panels, 128-column blocks, one to several CTAs per panel;
+32-row quarters of the triangles), through the star product's inverse, on matrices
 whose pivots leave the diagonal."""
 import numpy as np
 import pytest
@@ -10,7 +11,8 @@ from oracle.smatrix_oracle import star_product
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,batch", [(129, 2), (143, 3), (144, 1), (145, 2), (255, 1), (257, 2), (400, 2), (513, 1),
+@pytest.mark.parametrize("n,batch", [(1, 2), (2, 1), (15, 2), (16, 2), (17, 3), (31, 2), (33, 2), (64, 1),
+                                     (98, 3), (115, 2), (116, 2), (117, 2), (129, 2), (143, 3), (144, 1), (145, 2), (255, 1), (257, 2), (400, 2), (513, 1),
                                      (529, 2), (1030, 1)])
 def test_star_product_inverse(n, batch):
     rng = np.random.default_rng(n)
