@@ -265,9 +265,11 @@ int rcwa_set_eig_cluster(int ctas);
  * from order 1024 on; smaller orders report 1. */
 int rcwa_eig_cluster_size(int n, int batch);
 /* The same for the panel step of the LU factorisations (interface and tau
- * factorisations, rcwa_zgetrf stages): a batch of large matrices (order >=
- * 1024) that would leave half of the SMs idle factorises each 32-column
- * panel on a cluster of up to 8 CTAs per matrix, with identical factors.
+ * factorisations, rcwa_zgetrf stages): a panel runs on a cluster of up to 8
+ * CTAs per matrix, with identical factors.  Up to order 4096 a panel takes a
+ * CTA per 512 rows, or the forced size if that is larger; above, the forced
+ * size or, for a batch that would leave half of the SMs idle, up to 8
+ * (rcwa_lu_cluster_size reports that rule's size from order 1024 on).
  * ctas = 0: automatic, 1..8: forced; RCWA_ERR_INVALID outside 0..8. */
 int rcwa_set_lu_cluster(int ctas);
 
