@@ -1772,10 +1772,13 @@ __global__ void __launch_bounds__(kHessThreads) hessenberg_kernel(cplx* const* A
   }
   ex = block_max_int(ex, redi) - 1023;
   const int sh = ex > 100 ? min(ex, 1000) : ex < -100 ? max(ex, -1000) : 0;
+  // no CTA writes the matrix before every CTA of the team has read all of it:
+  // the reduction's first column can cross the bound that the scan tests, and
+  // the CTAs must agree on the branch below, which holds a barrier
+  if (kTeam) tm.sync();
   if (sh != 0) {
     const double f = scalbn(1.0, -sh);
     const int per = (n + tm.size - 1) / tm.size;
-    tm.sync();  // every CTA has read the matrix
     for (int i = tm.rank * per; i < min(n, (tm.rank + 1) * per); ++i)
       for (int j = threadIdx.x; j < n; j += blockDim.x) A[(size_t)i * lda + j] = cscale(A[(size_t)i * lda + j], f);
     tm.sync();

@@ -42,6 +42,28 @@ def test_team_sizes_give_identical_results(eng, n, b):
         assert res < 1e-11
 
 
+@pytest.mark.parametrize("log2max", [100.9, 101.1, -99.9, -100.1])
+def test_teams_agree_beside_the_scaling_bounds(eng, log2max):
+    # the reduction scales a matrix whose largest component has an exponent
+    # outside [-100, 100]; at 100.9 it does not, but the first reflector's beta
+    # (the norm of a column) lies above the bound, so a CTA that still scanned
+    # after the first one had written beta would decide otherwise
+    n = 200
+    A = _matrices(n, 2, 11)
+    A *= 2.0 ** log2max / max(np.abs(A.real).max(), np.abs(A.imag).max())
+    o.set_eig_cluster(1)
+    w1, V1, i1 = eng.zgeev(A)
+    for team in (2, 8):
+        o.set_eig_cluster(team)
+        w, V, info = eng.zgeev(A)
+        assert np.array_equal(info, i1) and np.array_equal(w, w1) and np.array_equal(V, V1), team
+    o.set_eig_cluster(0)
+    assert not np.any(i1)
+    # backward error of a QR iteration: a modest multiple of n u |A|
+    for k in range(2):
+        assert np.linalg.norm(A[k] @ V1[k] - V1[k] * w1[k]) <= 40 * n * 2.0 ** -53 * np.linalg.norm(A[k])
+
+
 def test_automatic_team_for_few_large_matrices(eng):
     o.set_eig_cluster(0)
     assert o.eig_cluster_size(882, 4) == 1        # below the order threshold
