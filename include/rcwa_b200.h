@@ -253,25 +253,27 @@ int rcwa_set_qr_sweep_limit(int sweeps);
 /* CTAs per matrix of the Hessenberg reduction and the multishift Schur
  * iteration (no reference counterpart: a scheduling choice of this engine).
  * A batch that would leave half of the SMs idle is given a thread-block
- * cluster of up to 8 CTAs per matrix (orders of at most 116, which run in
- * shared memory, one CTA); every element is computed by the same operations whatever the team size, so the
- * results are identical.  ctas = 0 restores the automatic choice, 1..8 forces
- * a size for every later eigensolve (matrices of order >= 64).  Process-wide;
- * a plan captured into a CUDA graph keeps the size chosen when it was
- * captured.  Returns RCWA_ERR_INVALID outside 0..8. */
+ * cluster of up to 8 CTAs per matrix; orders of at most 116, which run in
+ * shared memory, always take one CTA.  Every element is computed by the same
+ * operations whatever the team size, so the results are identical.  ctas = 0
+ * restores the automatic choice, 1..8 forces a size for every later eigensolve
+ * outside shared memory.  Process-wide; a plan captured into a CUDA graph keeps
+ * the size chosen when it was captured.  Returns RCWA_ERR_INVALID outside 0..8. */
 int rcwa_set_eig_cluster(int ctas);
-/* The team size rcwa_set_eig_cluster's setting gives a batch of `batch`
- * order-n matrices on the current device.  The automatic choice is reported
- * from order 1024 on; smaller orders report 1. */
+/* The team size an eigensolve of `batch` order-n matrices takes on the current
+ * device with the present setting (and the built-in Schur crossover). */
 int rcwa_eig_cluster_size(int n, int batch);
 /* The same for the panel step of the LU factorisations (interface and tau
- * factorisations, rcwa_zgetrf stages): a panel runs on a cluster of up to 8
- * CTAs per matrix, with identical factors.  Up to order 4096 a panel takes a
- * CTA per 512 rows, or the forced size if that is larger; above, the forced
- * size or, for a batch that would leave half of the SMs idle, up to 8
- * (rcwa_lu_cluster_size reports that rule's size from order 1024 on).
- * ctas = 0: automatic, 1..8: forced; RCWA_ERR_INVALID outside 0..8. */
+ * factorisations): a panel runs on a cluster of up to 8 CTAs per matrix, with
+ * identical factors.  Up to order 4096 a panel takes a CTA per 512 rows, or the
+ * forced size if that is larger; above, the forced size or, for a batch that
+ * would leave half of the SMs idle, up to 8.  ctas = 0: automatic, 1..8:
+ * forced; RCWA_ERR_INVALID outside 0..8. */
 int rcwa_set_lu_cluster(int ctas);
+/* The CTAs per matrix of the first (tallest) panel of an FP64 factorisation of
+ * `batch` order-n matrices under the built-in schedule rule; 1 where that rule
+ * gives each whole matrix to one CTA. */
+int rcwa_lu_cluster_size(int n, int batch);
 
 /* Fields inside a solved stack, for one point of an executed single-chunk
  * plan: the mode amplitudes of every interior layer for the plane wave
@@ -290,7 +292,6 @@ int rcwa_set_lu_cluster(int ctas);
 int rcwa_plan_field_rows(const rcwa_plan* plan, int point, int slice, int nres1, int* rows);
 int rcwa_plan_field(rcwa_plan* plan, int point, rcwa_cplx px, rcwa_cplx py, int slice, double coord,
                     int component, int nres1, rcwa_cplx* field);
-int rcwa_lu_cluster_size(int n, int batch);
 
 /* Batched complex GEMM D = alpha*A*B + beta*C (row-major, host buffers
  * [batch][M*K], [batch][K*N], [batch][M*N]; C may be NULL when beta = 0), the

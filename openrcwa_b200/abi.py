@@ -211,7 +211,7 @@ def set_eig_cluster(ctas: int) -> None:
 
 
 def eig_cluster_size(n: int, batch: int) -> int:
-    """The team size the current setting gives a batch of order-n matrices."""
+    """The CTAs per matrix an eigensolve of `batch` order-n matrices takes."""
     return int(load().rcwa_eig_cluster_size(int(n), int(batch)))
 
 
@@ -223,7 +223,8 @@ def set_lu_cluster(ctas: int) -> None:
 
 
 def lu_cluster_size(n: int, batch: int) -> int:
-    """The LU panel team size the current setting gives a batch of order-n matrices."""
+    """The CTAs per matrix of the first panel of an FP64 LU of `batch` order-n
+    matrices under the built-in schedule rule."""
     return int(load().rcwa_lu_cluster_size(int(n), int(batch)))
 
 

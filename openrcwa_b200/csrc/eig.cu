@@ -1847,10 +1847,6 @@ std::atomic<int> g_qr_sweep_cap{0};
 // automatic choice), set by rcwa_set_eig_cluster.
 std::atomic<int> g_eig_team{0};
 
-// rcwa_eig_cluster_size reports the automatic team of orders from here on
-// (smaller ones report 1; their launches choose by the same rule).
-constexpr int kTeamMinN = 1024;
-
 // Clusters of `size` CTAs of `kernel` that fit on the device at once.
 template <class K>
 int active_clusters(K kernel, int threads, size_t smem, int size) {
@@ -1873,6 +1869,12 @@ int active_clusters(K kernel, int threads, size_t smem, int size) {
   return nc;
 }
 
+// Allows the multishift kernel its dynamic shared memory on this device.
+cudaError_t schur_ms_ready() {
+  static SmemAttrOnce attr;
+  return attr.ensure(schur_ms_kernel, (int)kMsSmemBytes);
+}
+
 // Team size for a batch of order-n matrices: the largest (up to 8, and a CTA
 // per 64 rows) whose clusters of both kernels all fit on the device in one
 // wave, when the batch alone would leave at least half of the SMs idle; 1
@@ -1881,7 +1883,8 @@ int eig_team_auto(int n, int batch) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (batch <= 0 || 2 * batch > sms) return 1;
+  // the occupancy of the Schur kernel needs its shared memory allowed first
+  if (batch <= 0 || 2 * batch > sms || schur_ms_ready() != cudaSuccess) return 1;
   const int most = std::min(std::min(8, sms / batch), std::max(1, n / 64));
   static std::mutex mu;
   static std::map<std::tuple<int, int, int>, int> cache;  // (device, batch, largest size) -> size
@@ -1898,6 +1901,18 @@ int eig_team_auto(int n, int batch) {
     }
   cache[key] = pick;
   return pick;
+}
+
+// Whether matrices of order n run the shared-memory Schur kernel at crossover
+// ms_min (0: the largest).
+bool in_shared_memory(int n, int ms_min) { return n <= kBlkMax && (ms_min <= 0 || n < std::max(ms_min, kMsMin)); }
+
+// CTAs per matrix of a batch of order-n matrices: one where the matrix is held
+// in shared memory, else the forced or the automatic team.
+int eig_team(int n, int batch, int ms_min) {
+  if (in_shared_memory(n, ms_min)) return 1;
+  const int forced = g_eig_team.load();
+  return forced > 0 ? forced : eig_team_auto(n, batch);
 }
 
 // launch of kernel over batch * team CTAs in clusters of `team`
@@ -1947,27 +1962,19 @@ extern "C" int rcwa_set_eig_cluster(int ctas) {
 }
 
 extern "C" int rcwa_eig_cluster_size(int n, int batch) {
-  if (n < kMsMin || batch <= 0) return 1;
-  const int forced = g_eig_team.load();
-  if (forced > 0) return forced;
-  return n < kTeamMinN ? 1 : eig_team_auto(n, batch);
+  return n <= 0 || batch <= 0 ? 1 : eig_team(n, batch, 0);
 }
 
 cudaError_t zgeev_batched(cplx* const* A, int n, int lda, cplx* w, cplx* const* VR, int ldv, void* work,
                           int* info, int batch, cudaStream_t st, StageProf* prof, int ms_min) {
   if (batch <= 0 || n <= 0) return cudaSuccess;
-  ms_min = ms_min <= 0 ? kBlkMax + 1 : max(ms_min, kMsMin);
   const int sweep_cap = g_qr_sweep_cap.load();
   StageProf none;
   StageProf& P = prof ? *prof : none;
-  static SmemAttrOnce attr;
-  cudaError_t e = attr.ensure(schur_ms_kernel, (int)kMsSmemBytes);
+  cudaError_t e = schur_ms_ready();
   if (e != cudaSuccess) return e;
-  // a team of CTAs per matrix where the batch is too small to fill the GPU
-  // (matrices held in shared memory always run one CTA)
-  const bool block = n < ms_min && n <= kBlkMax;
-  const int forced = g_eig_team.load();
-  const int team = block ? 1 : forced > 0 ? forced : eig_team_auto(n, batch);
+  const bool block = in_shared_memory(n, ms_min);
+  const int team = eig_team(n, batch, ms_min);
   e = team > 1 ? launch_team(hessenberg_kernel<true>, batch, team, kHessThreads, 0, st, A, n, lda, work)
                : launch_team(hessenberg_kernel<false>, batch, 1, kHessThreads, 0, st, A, n, lda, work);
   if (e != cudaSuccess) return e;

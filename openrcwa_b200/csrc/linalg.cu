@@ -943,12 +943,17 @@ cudaError_t launch_panel(cplx* const* A, int n, int lda, int kb, int jb, int* ip
 }  // namespace
 
 namespace {
-// A register panel on the CTAs its rows need (or the forced cluster size).
+// Threads of a register panel of `rows` rows (one per row), and its CTAs: what
+// its rows need, or the forced cluster size if that is larger.
+int regpanel_threads(int rows) { return rows <= 128 ? 128 : rows <= 256 ? 256 : kRegT; }
+int regpanel_team(int rows) {
+  const int threads = regpanel_threads(rows);
+  return std::max((rows + threads - 1) / threads, g_lu_team.load());
+}
+
 cudaError_t launch_regpanel(cplx* const* A, int n, int lda, int kb, int jb, int* ipiv, int* info, int batch,
                             cudaStream_t st) {
-  const int rows = n - kb;
-  const int threads = rows <= 128 ? 128 : rows <= 256 ? 256 : kRegT;
-  const int team = std::max((rows + threads - 1) / threads, g_lu_team.load());
+  const int threads = regpanel_threads(n - kb), team = regpanel_team(n - kb);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(batch * team);
   cfg.blockDim = dim3(threads);
@@ -985,8 +990,8 @@ extern "C" int rcwa_set_lu_cluster(int ctas) {
 }
 
 extern "C" int rcwa_lu_cluster_size(int n, int batch) {
-  if (batch <= 0 || n <= 0) return 1;
-  return lu_team_size(n, batch);
+  if (batch <= 0 || n <= 0 || zgetrf_default_schedule(n, batch) == 0) return 1;
+  return n <= kRegMaxRows ? regpanel_team(n) : lu_team_size(n, batch);
 }
 
 int zgetrf_default_schedule(int n, int batch, int sms) {

@@ -66,8 +66,10 @@ def test_teams_agree_beside_the_scaling_bounds(eng, log2max):
 
 def test_automatic_team_for_few_large_matrices(eng):
     o.set_eig_cluster(0)
-    assert o.eig_cluster_size(882, 4) == 1        # below the order threshold
+    assert 2 <= o.eig_cluster_size(882, 4) <= 8
+    assert o.eig_cluster_size(200, 4) == 3        # a CTA per 64 rows
     assert o.eig_cluster_size(1200, 148) == 1     # the batch fills the GPU
+    assert o.eig_cluster_size(116, 4) == 1        # held in shared memory
     team = o.eig_cluster_size(1200, 4)
     assert 2 <= team <= 8
     A = _matrices(1200, 4, 7)
@@ -76,6 +78,37 @@ def test_automatic_team_for_few_large_matrices(eng):
     w1, V1, _ = eng.zgeev(A)
     o.set_eig_cluster(0)
     assert np.array_equal(w, w1) and np.array_equal(V, V1)
+
+
+def test_reported_sizes_are_those_of_the_launches(eng):
+    # orders in shared memory take one CTA whatever is forced
+    o.set_eig_cluster(8)
+    try:
+        assert [o.eig_cluster_size(n, 4) for n in (14, 64, 116, 117)] == [1, 1, 1, 8]
+    finally:
+        o.set_eig_cluster(0)
+    # LU: one CTA for the whole matrix, then a CTA per 512 rows of the first
+    # panel, or the forced size if that is larger
+    o.set_lu_cluster(0)
+    assert [o.lu_cluster_size(n, 2) for n in (98, 128, 200, 512, 513, 1058, 4096)] == [1, 1, 1, 1, 2, 3, 8]
+    assert o.lu_cluster_size(882, 1200) == 1
+    o.set_lu_cluster(2)
+    try:
+        assert [o.lu_cluster_size(n, 2) for n in (98, 200, 1058, 4097)] == [1, 2, 3, 2]
+    finally:
+        o.set_lu_cluster(0)
+
+
+def test_team_size_asked_before_the_first_solve():
+    # the query must not depend on (or, being kept, spoil) what a solve sets up
+    import subprocess
+    import sys
+    code = ("import openrcwa_b200 as o; a = o.eig_cluster_size(882, 4); e = o.Engine(0); "
+            "import numpy as np; e.zgeev(np.eye(130)[None] + 0j); print(a, o.eig_cluster_size(882, 4))")
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    a, b = (int(x) for x in out.stdout.split())
+    assert a == b and a >= 2
 
 
 def test_solve_with_teams_matches_single_cta(eng):
