@@ -1057,19 +1057,33 @@ cudaError_t zgetrf_columns(cplx* const* A, int n, int lda, int k0, int ce, int* 
   return cudaGetLastError();
 }
 
-// From this order and this many right-hand sides on, solves run blocked
-// (lu_blocked.cu: 128-row triangles with a thread per right-hand side and the
-// entries of 32 rows in registers, plus batched GEMM updates over the whole
-// grid) instead of one CTA per 64-column slab, whose triangles wait for a
-// dependent load per entry (B200, interface solves of 600 x 58 1.43 -> 0.63 ms,
-// 400 x 98 3.32 -> 1.75 ms, 200 x 198 7.05 -> 2.76 ms).  Below 16 a quarter's
-// 32 rows are mostly padding.
+// Whether a solve runs blocked (lu_blocked.cu: 128-row triangles with a thread
+// per right-hand side and the entries of 32 rows in registers, plus batched
+// GEMM updates over the whole grid) or on one CTA per 64-column slab, whose
+// triangles wait for a dependent load per entry.  Callers have 1, 2 or at least
+// n right-hand sides; for 1 or 2 most of a blocked CTA would be idle.  With more
+// slabs than SMs the blocked route is faster at every order from 16 on (B200,
+// solves of 300 x 16 1.7x, 1200 x 22 4.2x, 148 x 98 1.6x, 300 x 126 1.9x), and
+// from order 129 on for one matrix too.  One wave of slabs of a single block
+// costs the slab kernel its n rows and the blocked one its padded rows of 32, so
+// it takes over within each 32 rows where they are filled, in the last ones
+// (97-128) not at all (B200, slab kernel's time over the blocked one's, one to
+// 74 matrices: 0.59-0.64 at order 16, 0.95-1.0 at 26, 1.0-1.08 at 28, 0.88-0.91
+// at 34, 0.95-1.01 at 42, 1.0-1.07 at 44, 0.93-0.97 at 66, 0.97-1.07 at 82,
+// 0.84-0.91 at 98, 0.95-1.04 at 128).
 constexpr int kBlockedSolveMin = 16;
+
+bool solve_blocked(int n, int nrhs, int batch) {
+  if (n < kBlockedSolveMin || nrhs < kBlockedSolveMin) return false;
+  if (n > 128 || (long long)batch * ((nrhs + 63) / 64) > sm_count()) return true;
+  constexpr int kFrom[4] = {27, 43, 80, 129};
+  return n >= kFrom[(n - 1) / 32];
+}
 
 cudaError_t zgetrs_batched(const cplx* const* LU, int n, int lda, const int* ipiv, cplx* const* B,
                            int nrhs, int ldb, int batch, cudaStream_t st) {
   if (batch <= 0 || n <= 0 || nrhs <= 0) return cudaSuccess;
-  if (n >= kBlockedSolveMin && nrhs >= kBlockedSolveMin)
+  if (solve_blocked(n, nrhs, batch))
     return zgetrs_blocked_batched(LU, n, lda, ipiv, B, nrhs, ldb, batch, false, nullptr, st);
   dim3 grid((nrhs + 63) / 64, batch);
   zgetrs_kernel<false><<<grid, kTileThreads, 0, st>>>(LU, n, lda, ipiv, B, nrhs, ldb);
@@ -1080,7 +1094,7 @@ cudaError_t zgetrs_batched(const cplx* const* LU, int n, int lda, const int* ipi
 cudaError_t zgetri_batched(const cplx* const* LU, int n, int lda, const int* ipiv, cplx* const* X, int ldx,
                            int batch, cudaStream_t st) {
   if (batch <= 0 || n <= 0) return cudaSuccess;
-  if (n >= kBlockedSolveMin) return zgetrs_blocked_batched(LU, n, lda, ipiv, X, n, ldx, batch, true, nullptr, st);
+  if (solve_blocked(n, n, batch)) return zgetrs_blocked_batched(LU, n, lda, ipiv, X, n, ldx, batch, true, nullptr, st);
   dim3 grid((n + 63) / 64, batch);
   zgetrs_kernel<true><<<grid, kTileThreads, 0, st>>>(LU, n, lda, ipiv, X, n, ldx);
   ++launch_counter();

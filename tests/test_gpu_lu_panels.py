@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,batch", [(1, 2), (2, 1), (15, 2), (16, 2), (17, 3), (31, 2), (33, 2), (64, 1),
                                      (98, 3), (115, 2), (116, 2), (117, 2), (129, 2), (143, 3), (144, 1), (145, 2), (255, 1), (257, 2), (400, 2), (513, 1),
-                                     (529, 2), (1030, 1)])
+                                     (529, 2), (1030, 1),
+                                     # more 64-column slabs than SMs: blocked solves at every order
+                                     (16, 149), (17, 149), (33, 149), (66, 75), (98, 75), (117, 75)])
 def test_star_product_inverse(n, batch):
     rng = np.random.default_rng(n)
 
