@@ -32,7 +32,7 @@ struct Scratch {
   cplx* Z;     // n*n, column-major: Z(r, c) = Z[c*n + r]
   cplx* X;     // n*n, row-major upper-triangular eigenvector matrix of T
   cplx* v;     // n: current Householder vector / work column
-  double* scale; // what the Schur form is to be multiplied with (n complex)
+  double* scale; // what the eigenvalues are to be multiplied with (n complex)
   cplx* uv;    // n
   cplx* v0;    // n: leading element of each stored reflector
   cplx* Vb;    // n x kHb  panel reflectors, explicit (row-major)
@@ -1649,16 +1649,8 @@ __global__ void __launch_bounds__(kMsThreads) schur_ms_kernel(cplx* const* Aarr,
 #endif
   if (tm.rank == 0) {
     const double f = s.scale[0];
-    if (f != 1.0) {
-      __syncthreads();
-      for (size_t idx = threadIdx.x; idx < (size_t)n * n; idx += blockDim.x) {
-        cplx* const v = A + (idx / n) * lda + idx % n;
-        *v = cscale(*v, f);
-      }
-      __syncthreads();
-    }
     cplx* w = w_all + (size_t)mb * n;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) w[k] = A[(size_t)k * lda + k];
+    for (int k = threadIdx.x; k < n; k += blockDim.x) w[k] = cscale(A[(size_t)k * lda + k], f);
     if (threadIdx.x == 0) info_all[mb] = status;
   }
 }
@@ -1757,9 +1749,10 @@ __global__ void __launch_bounds__(kHessThreads) hessenberg_kernel(cplx* const* A
   const int mb = blockIdx.x / tm.size;
   const Scratch s = scratch_for(work, n, mb);
   cplx* A = Aarr[mb];
-  // a matrix whose products could leave the normal range is reduced and
-  // iterated at a power of two of its size (exact); the Schur kernel scales
-  // its result back
+  // a matrix whose products could leave the normal range is reduced, iterated
+  // and back-substituted at a power of two of its size (exact; a scaled-back
+  // Schur form could overflow, or lie below the smallest divisor that the back
+  // substitution allows); only the eigenvalues are scaled back
   int ex = 0;
   for (int i = threadIdx.x >> 5; i < n; i += blockDim.x >> 5) {
     int e4 = 0;
@@ -1805,13 +1798,13 @@ __global__ void __launch_bounds__(kBlkThreads) schur_block_kernel(cplx* const* A
     __syncthreads();
     status = schur_block<Q>(T, ld, s.Z, n, sweep_cap);
     __syncthreads();
-    const double f = s.scale[0];
     for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x)
-      A[(size_t)(idx / n) * lda + idx % n] = cscale(T[(idx / n) * ld + idx % n], f);
+      A[(size_t)(idx / n) * lda + idx % n] = T[(idx / n) * ld + idx % n];
     __syncthreads();
   }
+  const double f = s.scale[0];
   cplx* w = w_all + (size_t)blockIdx.x * n;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) w[k] = A[(size_t)k * lda + k];
+  for (int k = threadIdx.x; k < n; k += blockDim.x) w[k] = cscale(A[(size_t)k * lda + k], f);
   if (threadIdx.x == 0) info_all[blockIdx.x] = status;
 }
 

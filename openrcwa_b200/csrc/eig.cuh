@@ -20,7 +20,8 @@ __host__ __device__ constexpr size_t zgeev_workspace_bytes(int n) {
 }
 
 // For every batch item: A (n x n row-major, destroyed: holds the Schur form on
-// return) -> w (n eigenvalues), VR (n x n row-major, column k the unit-norm
+// return, times a power of two where the largest component's exponent lies
+// outside [-100, 100]) -> w (n eigenvalues), VR (n x n row-major, column k the unit-norm
 // right eigenvector of w[k]).  work: batch * zgeev_workspace_bytes(n) bytes.
 // info[b] = 0, or RCWA_ERR_NOCONV / RCWA_ERR_NONFINITE.  ms_min: the Schur
 // crossover (matrices below it that fit in shared memory run the block

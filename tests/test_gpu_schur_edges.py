@@ -19,22 +19,32 @@ def _cases(n, rng):
     if n > 2:
         H[n // 2, n // 2 - 1] = 0.0                              # already reducible
     yield H
-    # scaled so that the reduction's sums of squares, 1e+-240 n^2, stay normal
-    # with their relative accuracy (at 1e-150 they are subnormal and the
-    # Householder reduction, which does not scale, loses digits)
-    yield R * 1e120
-    yield R * 1e-120
     yield np.zeros((n, n), dtype=complex)
+
+
+def _scales(R):
+    # a matrix whose largest component's exponent lies outside [-100, 100] is
+    # reduced, iterated and back-substituted at a power of two of its size: just
+    # inside and outside the bounds, and to the ends of the range, where products
+    # of the entries leave it and (at 1e-300) the entries lie below LAPACK's
+    # smallest divisor of the back substitution
+    top = max(np.abs(R.real).max(), np.abs(R.imag).max())
+    yield from (2.0 ** 100.9 / top, 2.0 ** 101.1 / top, 2.0 ** -99.9 / top, 2.0 ** -100.1 / top)
+    yield from (1e120, 1e-120, 1e150, 1e-150, 1e300, 1e-300)
 
 
 @pytest.mark.parametrize("n", [1, 2, 3, 4, 7, 8, 31, 32, 33, 63, 64, 65, 96, 97, 115, 116, 117, 129, 150])
 def test_schur_edges(n):
-    A = np.array(list(_cases(n, np.random.default_rng(n))))
+    rng = np.random.default_rng(n)
+    A = list(_cases(n, rng))
+    R = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    scale = np.array([1.0] * len(A) + list(_scales(R)))
+    A = np.array(A + [R] * (len(scale) - len(A)))
     eng = o.Engine(0)
-    w, V, info = eng.zgeev(A)
+    w, V, info = eng.zgeev(A * scale[:, None, None])
     eng.close()
     assert not np.any(info)
-    for a, ww, v in zip(A, w, V):
+    for a, ww, v in zip(A, w / scale[:, None], V):
         # backward error of a QR iteration: a modest multiple of n u |A|
         assert np.linalg.norm(a @ v - v * ww) <= 40 * n * 2.0 ** -53 * max(np.linalg.norm(a), 1e-300)
         assert np.allclose(np.linalg.norm(v, axis=0), 1.0, atol=1e-12)
