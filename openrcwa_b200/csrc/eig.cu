@@ -1896,14 +1896,10 @@ int eig_team_auto(int n, int batch) {
   return pick;
 }
 
-// Whether matrices of order n run the shared-memory Schur kernel at crossover
-// ms_min (0: the largest).
-bool in_shared_memory(int n, int ms_min) { return n <= kBlkMax && (ms_min <= 0 || n < std::max(ms_min, kMsMin)); }
-
 // CTAs per matrix of a batch of order-n matrices: one where the matrix is held
 // in shared memory, else the forced or the automatic team.
 int eig_team(int n, int batch, int ms_min) {
-  if (in_shared_memory(n, ms_min)) return 1;
+  if (zgeev_in_shared_memory(n, ms_min)) return 1;
   const int forced = g_eig_team.load();
   return forced > 0 ? forced : eig_team_auto(n, batch);
 }
@@ -1942,6 +1938,10 @@ cudaError_t launch_block(cplx* const* A, int n, int lda, cplx* w, void* work, in
 
 }  // namespace
 
+bool zgeev_in_shared_memory(int n, int ms_min) {
+  return n <= kBlkMax && (ms_min <= 0 || n < std::max(ms_min, kMsMin));
+}
+
 extern "C" int rcwa_set_qr_sweep_limit(int sweeps) {
   if (sweeps < 0) return RCWA_ERR_INVALID;
   g_qr_sweep_cap.store(sweeps);
@@ -1966,7 +1966,7 @@ cudaError_t zgeev_batched(cplx* const* A, int n, int lda, cplx* w, cplx* const* 
   StageProf& P = prof ? *prof : none;
   cudaError_t e = schur_ms_ready();
   if (e != cudaSuccess) return e;
-  const bool block = in_shared_memory(n, ms_min);
+  const bool block = zgeev_in_shared_memory(n, ms_min);
   const int team = eig_team(n, batch, ms_min);
   e = team > 1 ? launch_team(hessenberg_kernel<true>, batch, team, kHessThreads, 0, st, A, n, lda, work)
                : launch_team(hessenberg_kernel<false>, batch, 1, kHessThreads, 0, st, A, n, lda, work);

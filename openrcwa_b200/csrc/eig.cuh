@@ -30,3 +30,8 @@ __host__ __device__ constexpr size_t zgeev_workspace_bytes(int n) {
 cudaError_t zgeev_batched(cplx* const* A, int n, int lda, cplx* w, cplx* const* VR, int ldv,
                           void* work, int* info, int batch, cudaStream_t st, StageProf* prof = nullptr,
                           int ms_min = 0);
+
+// Whether matrices of order n run the shared-memory Schur kernel at crossover
+// ms_min (0: every matrix that fits): crossovers that agree here launch the
+// same kernels.
+bool zgeev_in_shared_memory(int n, int ms_min);

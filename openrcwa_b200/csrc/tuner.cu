@@ -107,10 +107,9 @@ int tune_candidates(int op, int n, int* out) {
       out[2] = 2;
       return 3;
     case kTuneSchur:
-      // the crossover only matters while small active blocks are a large part
-      // of the iteration; from 512 rows on the multishift phase dominates
-      // (measured on B200: 64 fastest at n = 450, 882 and 1250), and a
-      // measurement there would cost seconds per candidate
+      // the crossover only decides between two kernels up to 116 rows; the
+      // other orders below 512 keep all four choices (tables hold them), each
+      // with the time of the one kernel they run
       if (n < kSchurCrossover || n >= kSchurTuneMax) { out[0] = kSchurCrossover; return 1; }
       for (int i = 0; i < kTuneMaxCand; ++i) out[i] = kSchurCand[i];
       return kTuneMaxCand;
@@ -198,6 +197,14 @@ cudaError_t tune_measure(rcwa_engine* e, int op, int n, int batch, TuneEntry& ou
     if ((err = fill(src.as<cplx>(), nn * mb, 0xE16ull + n, st)) != cudaSuccess) return err;
     auto restore = [&]() { return cudaMemcpyAsync(a.p, src.p, per * mb, cudaMemcpyDeviceToDevice, st); };
     for (int c = 0; c < out.ncand; ++c) {
+      // a candidate that launches the kernels of an earlier one has its time
+      // (a second run would differ by noise only, and decide by it)
+      int same = 0;
+      while (same < c && zgeev_in_shared_memory(n, out.cand[same]) != zgeev_in_shared_memory(n, out.cand[c])) ++same;
+      if (same < c) {
+        out.ms[c] = out.ms[same];
+        continue;
+      }
       auto run = [&](int b) {
         return zgeev_batched(pa.as<cplx*>(), n, n, w.as<cplx>(), pv.as<cplx*>(), n, wk.p, info.as<int>(), b, st,
                              nullptr, out.cand[c]);

@@ -45,6 +45,17 @@ def test_measure_returns_a_timed_candidate(eng, op, n, batch):
     t.close()
 
 
+@pytest.mark.parametrize("n,kernels", [(80, [[64], [96, 128, 192]]), (98, [[64, 96], [128, 192]]),
+                                       (130, [[64, 96, 128, 192]])])
+def test_crossovers_of_one_kernel_share_its_time(eng, n, kernels):
+    # choices that launch the same kernels must not be ranked by noise
+    t = o.Tuner()
+    choice, ms = t.measure(eng, "schur", n, 4)
+    assert all(len({ms[c] for c in k}) == 1 for k in kernels)
+    assert choice in [k[0] for k in kernels]   # the first of the fastest
+    t.close()
+
+
 @pytest.mark.parametrize("lu", [0, 1])
 @pytest.mark.parametrize("cross", [64, 96, 128, 192])
 def test_every_schedule_matches_oracle(eng, case, lu, cross):
