@@ -1072,13 +1072,6 @@ int plan_create_impl(rcwa_engine* e, const std::vector<StackInfo>& si, const rcw
         tdd[lp] = W_(c.Tdd) + nn * lp;
         gbuf[lp] = W_(c.G) + nn * lp;
       }
-      const size_t oR0 = meta.add_vec(rud), oT0 = meta.add_vec(tdd);
-      P->steps.push_back([=](cudaStream_t st, StageProf& pf) {
-        cudaError_t err = cascade_init((cplx* const*)((char*)plan->meta.p + oR0),
-                                       (cplx* const*)((char*)plan->meta.p + oT0), n, np, st);
-        pf.mark(st, kStPhase);
-        return err;
-      });
       // layer buffers of point lp, layer l
       auto layerW = [&](int lp, int l) -> cplx* {
         const int p = c.points[lp];
@@ -1265,9 +1258,10 @@ int plan_create_impl(rcwa_engine* e, const std::vector<StackInfo>& si, const rcw
           g.batch = k;
           g.gammaI = mkc(0, 0);
           // F = IE + IE waveRud ; G = IH - IH waveRud   (:440-443).  On the
-          // first step Rud = 0 and Tdd = I, so F = IE, G = IH and, below,
-          // Tdd = 2 tau without their products (148 one-layer points of order
-          // 450, FP64: products 32.1 -> 20.2 ms on B200)
+          // first step Rud = 0 and Tdd = I (their buffers are written there, not
+          // read), so F = IE, G = IH and, below, Tdd = 2 tau without their
+          // products (148 one-layer points of order 450, FP64: products 31.7 ->
+          // 20.0 ms on B200)
           if (step > 0) {
             g.A = cpa(ofA); g.B = cpa(ofB); g.C = cpa(ofC); g.D = pa(ofD);
             g.alpha = mkc(1, 0); g.beta = mkc(1, 0);
