@@ -113,18 +113,19 @@ def test_team_size_asked_before_the_first_solve():
 
 def test_solve_with_teams_matches_single_cta(eng):
     # one point of a 2D pillar grating at Nx = Ny = 11 (n = 1058): three layer
-    # eigensolves and LU batches of one and two matrices, so the automatic
-    # rule gives the eigensolver and the LU panels clusters of CTAs; R, T and
-    # every order must equal the one-CTA solve bit for bit
+    # eigensolves with automatic teams and LU panels on the three CTAs they
+    # need, against one CTA per eigensolve and panels forced to eight; R, T and
+    # every order must agree bit for bit
     from openrcwa_b200 import workloads
     stacks, pts, pxy = workloads.pillars_2d(seed=3, nH=11, n_lambda=1, n_angle=1, n_layers=3)
     o.set_eig_cluster(0)
     o.set_lu_cluster(0)
-    assert o.eig_cluster_size(1058, 3) > 1 and o.lu_cluster_size(1058, 1) > 1
+    assert o.eig_cluster_size(1058, 3) > 1 and o.lu_cluster_size(1058, 1) == 3
     R, T, REF, TRN, st = eng.solve_batch(stacks, pts[:1], pxy[:1])
     o.set_eig_cluster(1)
-    o.set_lu_cluster(1)
+    o.set_lu_cluster(8)
     try:
+        assert o.lu_cluster_size(1058, 1) == 8
         R1, T1, REF1, TRN1, st1 = eng.solve_batch(stacks, pts[:1], pxy[:1])
     finally:
         o.set_eig_cluster(0)

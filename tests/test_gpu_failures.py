@@ -47,7 +47,7 @@ def test_nan_permittivity_is_rejected_before_any_launch(eng):
 
 def test_nan_matrix_reports_nonfinite_from_the_eigensolver(eng):
     rng = np.random.default_rng(3)
-    for n in (30, 100):   # single-shift and multishift Schur kernels
+    for n in (30, 100, 150):   # shared-memory Schur kernel; multishift, a team of CTAs per matrix
         A = rng.normal(size=(3, n, n)) + 1j * rng.normal(size=(3, n, n))
         A[1, n // 2, n // 3] = complex(float("nan"), 1.0)
         w, VR, info = eng.zgeev(A)
@@ -85,7 +85,7 @@ def test_qr_sweep_cap_reports_noconv_and_resets(eng):
     st, pts, pxy = _small_2d()
     try:
         o.set_qr_sweep_limit(1)
-        for n in (30, 100):
+        for n in (30, 100, 150):
             A = rng.normal(size=(2, n, n)) + 1j * rng.normal(size=(2, n, n))
             _, _, info = eng.zgeev(A)
             assert np.all(info == abi.RCWA_ERR_NOCONV), info

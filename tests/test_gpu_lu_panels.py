@@ -11,6 +11,57 @@ from oracle.smatrix_oracle import star_product
 pytestmark = pytest.mark.gpu
 
 
+def _inverses(eng, A):
+    """(I - A)^-1 of every item, through the star product's Tdd with unit Tdd, Rud and tdd."""
+    I, Z = np.broadcast_to(np.eye(A.shape[-1], dtype=complex), A.shape), np.zeros_like(A)
+    got, st = eng.star_product({"Rud": I, "Rdu": Z, "Tdd": I, "Tuu": Z}, {"rud": Z, "rdu": A, "tdd": I, "tuu": Z})
+    assert not np.any(st)
+    return got["Tdd"]
+
+
+# one, two and three CTAs per first panel as the rows need them
+@pytest.mark.parametrize("n", [200, 529, 1058])
+def test_panel_clusters_give_identical_factors(n):
+    rng = np.random.default_rng(n)
+    A = (rng.standard_normal((2, n, n)) + 1j * rng.standard_normal((2, n, n))) / np.sqrt(n)
+    eng = o.Engine(0)
+    try:
+        o.set_lu_cluster(0)
+        X = _inverses(eng, A)
+        for team in (4, 8):
+            o.set_lu_cluster(team)
+            assert o.lu_cluster_size(n, 2) == team
+            assert np.array_equal(_inverses(eng, A), X), team
+    finally:
+        o.set_lu_cluster(0)
+        eng.close()
+    res = np.linalg.norm((np.eye(n) - A) @ X - np.eye(n)) / np.linalg.norm(X)
+    # residual of an inverse from an LU: a modest multiple of n u |A| |X|
+    assert res <= 40 * n * 2.0 ** -53 * np.linalg.norm(np.eye(n) - A)
+
+
+def test_panels_above_the_register_rows():
+    # above 4096 rows: 32-column panels updated in L2, by one CTA and by a team
+    n = 4101
+    rng = np.random.default_rng(7)
+    A = (rng.standard_normal((1, n, n)) + 1j * rng.standard_normal((1, n, n))) / np.sqrt(n)
+    eng = o.Engine(0)
+    try:
+        o.set_lu_cluster(1)
+        X = _inverses(eng, A)
+        o.set_lu_cluster(0)
+        assert o.lu_cluster_size(n, 1) > 1
+        assert np.array_equal(_inverses(eng, A), X)
+    finally:
+        o.set_lu_cluster(0)
+        eng.close()
+    v = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    x = X[0] @ v
+    # residual bound of a solve: a modest multiple of n u |A| |x|
+    norm_a = np.linalg.norm(np.eye(n) - A[0])
+    assert np.linalg.norm(x - A[0] @ x - v) <= 40 * n * 2.0 ** -53 * norm_a * np.linalg.norm(x)
+
+
 @pytest.mark.parametrize("n,batch", [(1, 2), (2, 1), (15, 2), (16, 2), (17, 3), (31, 2), (33, 2), (64, 1),
                                      (98, 3), (115, 2), (116, 2), (117, 2), (129, 2), (143, 3), (144, 1), (145, 2), (255, 1), (257, 2), (400, 2), (513, 1),
                                      (529, 2), (1030, 1),

@@ -179,8 +179,8 @@ def test_auto_mode_records_and_stays_exact(eng, case, tmp_path):
 
 @pytest.mark.parametrize("cross", [64, 128])
 def test_small_matrix_schur_paths(eng, cross):
-    # n = 98: multishift kernel (64) or the single-shift kernel for the whole
-    # matrix (128, the built-in rule below 128 rows)
+    # n = 98: multishift kernel (64) or the shared-memory kernel (128, the
+    # built-in rule below 128 rows)
     st, pts, pxy, ref = _stack_points(_setup(12, 3))
     n = 2 * st.N
     t = o.Tuner()

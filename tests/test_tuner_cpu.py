@@ -23,8 +23,8 @@ def test_candidates(tuner):
     assert t.candidates("lu", 200) == [0, 1]
     assert t.candidates("product", 98) == [0, 1, 2]
     assert t.candidates("schur", 242) == [64, 96, 128, 192]
-    assert t.candidates("schur", 882) == [64]  # large matrices: multishift phase dominates
-    assert t.candidates("schur", 40) == [64]   # below the crossover: single-shift only
+    assert t.candidates("schur", 882) == [64]  # not tuned from 512 rows on
+    assert t.candidates("schur", 40) == [64]   # always in shared memory
     with pytest.raises(o.RcwaError):
         t.candidates(7, 100)
 
@@ -39,7 +39,7 @@ def test_default_rules(tuner):
     assert t.default("lu", 882, 592) == 0
     assert t.default("lu", 128, 10) == 0
     assert t.default("schur", 882, 740) == 64
-    assert t.default("schur", 98, 200) == 128   # small matrices: single-shift kernel
+    assert t.default("schur", 98, 200) == 128   # small matrices: shared-memory kernel
     assert t.default("schur", 40, 200) == 64    # the only candidate below 64 rows
     assert t.default("product", 882, 148) == 0
     t.set_sms(100)
