@@ -864,8 +864,7 @@ cudaError_t zgemm_batched(const GemmArgs& g, cudaStream_t st) {
   return g.transB ? zgemm_launch<false, true>(g, st) : zgemm_launch<false, false>(g, st);
 }
 
-namespace {
-int sm_count() {
+int device_sm_count() {
   static int count = 0;
   if (!count) {
     int dev = 0, c = 0;
@@ -877,7 +876,6 @@ int sm_count() {
   }
   return count;
 }
-}  // namespace
 
 namespace {
 // CTAs per matrix of the multi-launch LU's panel step (0: automatic), set by
@@ -888,7 +886,7 @@ constexpr int kLuTeamMinN = 1024;
 int lu_team_size(int n, int batch) {
   const int forced = g_lu_team.load();
   if (forced > 0) return forced;
-  const int sms = sm_count();
+  const int sms = device_sm_count();
   if (n < kLuTeamMinN || 2 * batch > sms) return 1;
   static std::mutex mu;
   static std::map<int, int> cache;  // batch -> size
@@ -995,7 +993,7 @@ extern "C" int rcwa_lu_cluster_size(int n, int batch) {
 }
 
 int zgetrf_default_schedule(int n, int batch, int sms) {
-  if (sms <= 0) sms = sm_count();
+  if (sms <= 0) sms = device_sm_count();
   // 128-column blocks from n = 256 on (measured on B200 against panel by panel:
   // 58 x 882 13.6 -> 8.9 ms, 148 x 450 5.4 -> 4.2 ms; 2 x 1250 5.2 -> 6.2 ms)
   if (n <= 128 || batch >= 4 * sms) return 0;
@@ -1063,21 +1061,22 @@ cudaError_t zgetrf_columns(cplx* const* A, int n, int lda, int k0, int ce, int* 
 // triangles wait for a dependent load per entry.  Callers have 1, 2 or at least
 // n right-hand sides; for 1 or 2 most of a blocked CTA would be idle.  With more
 // slabs than SMs the blocked route is faster at every order from 16 on (B200,
-// solves of 300 x 16 1.7x, 1200 x 22 4.2x, 148 x 98 1.6x, 300 x 126 1.9x), and
-// from order 129 on for one matrix too.  One wave of slabs of a single block
-// costs the slab kernel its n rows and the blocked one its padded rows of 32, so
-// it takes over within each 32 rows where they are filled, in the last ones
-// (97-128) not at all (B200, slab kernel's time over the blocked one's, one to
-// 74 matrices: 0.59-0.64 at order 16, 0.95-1.0 at 26, 1.0-1.08 at 28, 0.88-0.91
-// at 34, 0.95-1.01 at 42, 1.0-1.07 at 44, 0.93-0.97 at 66, 0.97-1.07 at 82,
-// 0.84-0.91 at 98, 0.95-1.04 at 128).
+// solves of 300 x 16 1.7x, 1200 x 22 4.2x, 148 x 98 1.6x, 300 x 126 1.9x).  One
+// wave of slabs costs the slab kernel its n rows and the blocked one triangles
+// padded to 32 rows, so it keeps the orders with the most padding (slab kernel's
+// time over the blocked one's, one to 74 matrices with n right-hand sides:
+// 0.63-0.68 at order 16, 0.88-0.92 at 22, 0.94-1.03 at 24, 1.13-1.22 at 28,
+// 0.92-0.99 at 34, 0.98-1.04 at 38, 1.2-1.26 at 50, 1.0-1.09 at 66, 0.96-1.04 at
+// 98, 1.14-1.23 at 128).  Above 128 right-hand sides the blocked route needs a
+// second CTA per matrix: with 2 n or 3 n of them 1.16 at 50, 0.93-0.97 at 66-82,
+// 1.1 at 86, 0.89-0.92 at 98-116, 0.95-1.07 at 122, 1.03-1.07 at 128.
 constexpr int kBlockedSolveMin = 16;
 
 bool solve_blocked(int n, int nrhs, int batch) {
   if (n < kBlockedSolveMin || nrhs < kBlockedSolveMin) return false;
-  if (n > 128 || (long long)batch * ((nrhs + 63) / 64) > sm_count()) return true;
-  constexpr int kFrom[4] = {27, 43, 80, 129};
-  return n >= kFrom[(n - 1) / 32];
+  if ((long long)batch * ((nrhs + 63) / 64) > device_sm_count()) return true;
+  if (n < 24) return false;
+  return nrhs <= 128 ? n <= 32 || n >= 38 : n <= 64 || (n > 82 && n <= 96) || n > 122;
 }
 
 cudaError_t zgetrs_batched(const cplx* const* LU, int n, int lda, const int* ipiv, cplx* const* B,

@@ -27,6 +27,9 @@ struct GemmArgs {
   int triB = 0;
 };
 
+// SMs of the device that was current at the first call (148 without one).
+int device_sm_count();
+
 // D = alpha*op(A)*diag(s)*op(B) + beta*C + gammaI*I for every batch item.
 cudaError_t zgemm_batched(const GemmArgs& g, cudaStream_t st);
 
