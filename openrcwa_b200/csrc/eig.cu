@@ -1,4 +1,5 @@
-// Batched complex eigensolver, one CTA per matrix, FP64 throughout:
+// Batched complex eigensolver, one CTA per matrix or (above 116 rows, where the
+// batch leaves SMs idle) a cluster of up to 8, FP64 throughout:
 //   1. Householder reduction to upper Hessenberg form, Q accumulated backwards;
 //   2. small-bulge multishift QR (Ahues-Tisseur deflation test, exceptional
 //      shifts after 10 sweeps) producing the Schur form T with Schur vectors Z:
@@ -781,7 +782,8 @@ __device__ int schur_block(cplx* T, int ld, cplx* Z, int n, int sweep_cap) {
 // register shift per step and the chase's rotations on ten threads the same
 // matrix took 404 ms.  Schur stage of whole batches (window 64 / 72 / 100, early
 // deflation 16): 145 x 882 335 / 325 / 372 ms, 148 x 450 80 / 78 / 89 ms; ten
-// shifts (the frame spills) 537 ms, six 468 ms at 145 x 882.
+// shifts (the frame spills) 537 ms, six 468 ms at 145 x 882.  As built (window
+// 72, early deflation 12) 330 and 77 ms.
 #ifndef RCWA_MS_WINDOW
 #define RCWA_MS_WINDOW 72
 #endif
@@ -903,8 +905,9 @@ __device__ void small_eigs_warp(cplx* B, int ldb, int s, cplx* out) {
 // The window's one-warp Schur form is serial, so a smaller window is cheaper
 // per call and deflates less: Schur stage with windows of 16 / 14 / 12 (64-row
 // chase window) 145 x 882 335 / 346 / 342 ms, 148 x 450 80 / 81 / 75 ms, 74 x
-// 198 19.6 / 18.8 / 16.3 ms; a 32-row window on all warps cut the sweeps by 20%
-// but cost 60 + 35 ms for its Schur form and reordering at order 882.
+// 198 19.6 / 18.8 / 16.3 ms; one size serves all orders, and 12 costs order 882
+// 2%.  A 32-row window on all warps cut the sweeps by 20% but cost 60 + 35 ms for
+// its Schur form and reordering at order 882.
 #ifndef RCWA_AED_WINDOW
 #define RCWA_AED_WINDOW 12
 #endif

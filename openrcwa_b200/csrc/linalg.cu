@@ -18,9 +18,10 @@
 namespace {
 
 // Output tiles of 64 x 64 by four warps of 32 x 32, two CTAs per SM; slabs of
-// 8 along K in four stages (83 KB).  Bound by the FP64 tensor pipe: a warp's 32
-// x 32 share issues 64 DMMAs (16 cycles each on its quarter of the SM) for 16
-// shared loads, and the cp.async stages take the loads off its path.  The
+// 8 along K in four stages (98,816 bytes).  Bound by the FP64 tensor pipe: per K-step of
+// 4 a warp's 32 x 32 share issues 64 DMMAs (16 cycles each on its quarter of the
+// SM) for eight 16-byte shared loads, and the cp.async stages take the global
+// loads off its path.  The
 // routine of tile.cuh, whose 16 x 32 share per warp waits for two barriers and
 // a register-to-shared transpose per slab, reached half of the pipe: on B200
 // (DMMA peak measured 36.4 TFLOP/s) 29 x 882^3 8.49 -> 5.00 ms (31.8 TFLOP/s),
@@ -239,8 +240,9 @@ __global__ void __launch_bounds__(kTileThreads) zgetrf_kernel(cplx* const* Aarr,
 // the warps' arg-max (three redux steps), two barriers, the reciprocal and the
 // update.  Whole factorisations (schedule 2) against 32-column panels updated
 // in L2, B200: 58 x 882 16.4 -> 8.9 ms, 46 x 494 5.3 -> 2.6 ms, 148 x 450 6.1 ->
-// 4.2 ms, 2 x 1250 12.1 -> 5.2 ms.  Same pivot rule and the same operations per entry as
-// lu_panel, so the panel's factors are the same for every cluster size.
+// 4.2 ms, 2 x 1250 12.3 -> 6.2 ms (5.1 in schedule 1).  Same pivot rule and the
+// same operations per entry as lu_panel, so the panel's factors are the same for
+// every cluster size.
 constexpr int kRegW = 16;
 constexpr int kRegT = 512;
 constexpr int kRegMaxRows = 8 * kRegT;
@@ -881,13 +883,14 @@ namespace {
 // CTAs per matrix of the multi-launch LU's panel step (0: automatic), set by
 // rcwa_set_lu_cluster.
 std::atomic<int> g_lu_team{0};
-constexpr int kLuTeamMinN = 1024;
 
-int lu_team_size(int n, int batch) {
+// Team of the panels above kRegMaxRows rows: the forced size, or up to 8 CTAs
+// where the batch would leave half of the SMs idle.
+int lu_team_size(int batch) {
   const int forced = g_lu_team.load();
   if (forced > 0) return forced;
   const int sms = device_sm_count();
-  if (n < kLuTeamMinN || 2 * batch > sms) return 1;
+  if (2 * batch > sms) return 1;
   static std::mutex mu;
   static std::map<int, int> cache;  // batch -> size
   std::lock_guard<std::mutex> lk(mu);
@@ -989,13 +992,19 @@ extern "C" int rcwa_set_lu_cluster(int ctas) {
 
 extern "C" int rcwa_lu_cluster_size(int n, int batch) {
   if (batch <= 0 || n <= 0 || zgetrf_default_schedule(n, batch) == 0) return 1;
-  return n <= kRegMaxRows ? regpanel_team(n) : lu_team_size(n, batch);
+  return n <= kRegMaxRows ? regpanel_team(n) : lu_team_size(batch);
 }
 
 int zgetrf_default_schedule(int n, int batch, int sms) {
   if (sms <= 0) sms = device_sm_count();
-  // 128-column blocks from n = 256 on (measured on B200 against panel by panel:
-  // 58 x 882 13.6 -> 8.9 ms, 148 x 450 5.4 -> 4.2 ms; 2 x 1250 5.2 -> 6.2 ms)
+  // The lines were drawn with the 32-column panels in L2 and hold for full
+  // batches (B200, schedules 1 / 2: 58 x 882 13.6 / 9.0 ms, 148 x 450 5.4 / 4.2,
+  // 148 x 256 1.35 / 1.25; 0 / 1: 148 x 98 0.17 / 0.30).  With the register
+  // panels schedule 1 is faster for few matrices (1 x 300 0.85 against 1.12 ms,
+  // 2 x 1250 5.1 against 6.2), for n = 117..128 (148 x 122 0.38 against 0.50) and,
+  // like schedule 2, for four waves and more (600 x 98 0.67 against 0.81, 600 x
+  // 198 2.6 against 5.9, 600 x 450 19.6 and 15.2 against 37.1); the tuner finds
+  // these.
   if (n <= 128 || batch >= 4 * sms) return 0;
   return n >= 256 ? 2 : 1;
 }
@@ -1039,7 +1048,7 @@ cudaError_t zgetrf_columns(cplx* const* A, int n, int lda, int k0, int ce, int* 
     return cudaSuccess;
   }
   // a cluster of CTAs per matrix shares each panel when the batch leaves SMs idle
-  const int team = lu_team_size(n, batch);
+  const int team = lu_team_size(batch);
   for (int kb = k0; kb < ce; kb += kLuPanel) {
     const int jb = min(kLuPanel, ce - kb);
     cudaError_t pe = launch_panel(A, n, lda, kb, jb, ipiv, info, batch, team, st);

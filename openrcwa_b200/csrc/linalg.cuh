@@ -36,7 +36,7 @@ cudaError_t zgemm_batched(const GemmArgs& g, cudaStream_t st);
 // In-place LU with partial pivoting (row interchanges, LAPACK getrf
 // convention, 0-based pivots) of square n x n matrices.  info[b] = 0, or k+1
 // when U(k,k) is exactly zero.  schedule 0: one CTA factors each matrix;
-// schedule 1: panel by panel, the panel factorisation one CTA per matrix and
+// schedule 1: panel by panel, the panel on the CTAs that its rows need and
 // the triangular solve and trailing update spread over all SMs; -1: the
 // default rule (zgetrf_default_schedule: schedule 0 for n <= 128 or batches of
 // at least four waves of CTAs, else 2 from n = 256 on, else 1; up to 116 rows
@@ -49,8 +49,8 @@ cudaError_t zgetrf_batched(cplx* const* A, int n, int lda, int* ipiv, int* info,
                            cudaStream_t st, int schedule = -1);
 // Columns k0 .. ce-1 of the panel-by-panel LU, whose columns before k0 are
 // factorised and whose columns from k0 on have taken every update of them:
-// 32-column panels (row interchanges across whole rows) with the U12 solves
-// and FP64 trailing updates confined to columns < ce.  The columns from ce on
+// 16-column panels (32 above 4096 rows; row interchanges across whole rows)
+// with the U12 solves and FP64 trailing updates confined to columns < ce.  The columns from ce on
 // are left to the caller (a blocked LU's trailing update).  k0 = 0 clears info.
 cudaError_t zgetrf_columns(cplx* const* A, int n, int lda, int k0, int ce, int* ipiv, int* info, int batch,
                            cudaStream_t st);

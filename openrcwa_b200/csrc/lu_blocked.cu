@@ -1,8 +1,8 @@
 // Blocked LU factorisation and solves with 128-wide blocks.
 //
 // The factorisation factors each 128-column block with the panel-by-panel LU
-// of linalg.cu confined to the block (zgetrf_columns: 32-column panels, row
-// interchanges across whole rows), solves the block row right of it against
+// of linalg.cu confined to the block (zgetrf_columns: 16-column panels, 32 above
+// 4096 rows, row interchanges across whole rows), solves the block row right of it against
 // the block's unit lower triangle, and updates the trailing matrix with one
 // batched product of K = 128.
 //

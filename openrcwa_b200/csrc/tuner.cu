@@ -122,8 +122,8 @@ int tune_default_sms(int op, int n, int batch, int sms) {
   switch (op) {
     case kTuneLU: return zgetrf_default_schedule(n, batch, sms);
     // up to 116 rows: the kernel that holds the matrix in shared memory
-    // (measured on B200, block against multishift kernel: 303 x 82 6.3 / 13.6
-    // ms, 400 x 98 17.2 / 21.1 ms)
+    // (whole eigensolves on B200, block against multishift kernel: 148 x 80 6.5 /
+    // 9.3 ms, 148 x 98 9.4 / 11.9 ms)
     case kTuneSchur: return (n >= kSchurCrossover && n < 128) ? 128 : kSchurCrossover;
     case kTuneProduct: return 0;
     default: return -1;

@@ -2,7 +2,7 @@
 // (matrix order, batch size class) it keeps the choice that ran fastest when
 // timed on this GPU.  Decisions:
 //   kTuneLU       LU factorisation schedule (0: one CTA per matrix, 1: panel
-//                 by panel over all SMs)
+//                 by panel over all SMs, 2: 128-column blocks)
 //   kTuneSchur    Schur crossover: matrices below it (and of at most 116
 //                 rows) are iterated in shared memory, others by windowed
 //                 multishift sweeps with early deflation
